@@ -123,7 +123,7 @@ def _fog(case, seed):
     sc = fog_scene.FogScene(fog_scene.fog_config(seed=int(seed) % 100000, width=case["w"], height=case["h"],
                                                  depth=case["d"]), "cuda")
     dt = torch.float16 if case["half"] else torch.float32
-    return [(sc.param_args(t), sc.inject(t, dt)) for t in range(3)]
+    return [(sc.param_args(t), sc.inject(t, dt)) for t in range(1, 4)]
 
 
 def _hdr(case, seed):
