@@ -1,32 +1,45 @@
 // Volumetric-fog froxel filter (include/tg_fog.h) on sm_103a.
 //
-// The reference's filterMain (src/volumetric_filter.slang:142-226).  A CTA
-// covers 32 x 4 columns of 8 consecutive slices, one thread per column: the
-// column's camera ray and the slices' view depths are computed once (they are
-// the same for every froxel of a column / slice), then for each slice the CTA
-// stages the 34 x 6 halo of injected texels in shared memory with coalesced
-// loads (the 3x3 mean reads shared memory; a texel is read from L2 once per CTA
-// instead of nine times) and each thread places its froxel centre on its ray,
-// projects it into the previous frame and fetches the history trilinearly.
+// The reference's filterMain (src/volumetric_filter.slang:142-226).  A CTA of 32 x 4
+// threads covers 32 x 8 columns of 8 consecutive slices, two vertically adjacent
+// columns per thread: the columns' camera rays and the slices' view depths are
+// computed once (they are the same for every froxel of a column / slice), then
+// for each slice the 34 x 10 halo of injected texels is staged in shared memory,
+// double-buffered (the next slice's texels are loaded while this slice is
+// computed, one barrier per slice), and each thread places its froxel centres on
+// their rays, projects them into the previous frame and fetches the history
+// trilinearly.
 //
-// Every add, multiply, divide and square root on the projection path is an
-// explicitly rounded IEEE operation (no contraction into FMA), in the order
-// the reference writes them, so the froxel coordinates that decide the
-// rejection tests and the trilinear weights are the reference's own float
-// arithmetic; only powf / logf (slice depth, its inverse) are CUDA's.
+// What bounds it: FP32 issue.  The compulsory traffic of a 320x180x64 rgba16f
+// pass (88 MB, L2-resident) is 13 us of the 6.8 TB/s a copy reaches.  Two columns
+// per thread share four rows of the 3x3 box (6 shared loads per froxel instead of
+// 9) and give two independent chains of projections and gathers.  Measured with
+// history: 79.9 us with one column per thread, two barriers per slice and a
+// division per quotient, 61.8 us as here.
+//
+// Every add, multiply, divide and square root on the projection path is rounded
+// as IEEE asks (no contraction into FMA), in the order the reference writes them,
+// so the froxel coordinates that decide the rejection tests and the trilinear
+// weights are the reference's own float arithmetic; only powf / logf (slice
+// depth, its inverse) are CUDA's.  Divisors are the same for a whole box, column,
+// froxel or launch, so quotients are formed by multiplying with the divisor's
+// correctly rounded reciprocal and correcting with FMA residuals, which rounds
+// correctly (Markstein 1990; Brisebarre, Muller and Raina 2004) while nothing
+// overflows or underflows; operands outside that range take the division itself.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
 
+#include "svgf_device.cuh"
 #include "svgf_internal.h"
 #include "tg_fog.h"
 
 namespace tg {
 namespace {
 
-// 128-thread CTAs: 4.6% faster per pass at 320x180x64 than 32 x 8 columns.
-constexpr int kFogTX = 32, kFogTY = 4;
+constexpr int kFogTX = 32, kFogRows = 4, kFogR = 2;  // threads across and down, columns (in y) per thread
+constexpr int kFogTY = kFogRows * kFogR;
 constexpr int kFogSW = kFogTX + 2, kFogSH = kFogTY + 2;
 constexpr int kFogZC = 8;  // slices per CTA
 
@@ -34,22 +47,36 @@ struct FogArgs {
     float ivp[16], pvp[16], cam[3];
     float alpha, znear, zfar;
     int W, H, D, valid;
+    int plain_div;  // the depth range is too extreme for quotients by reciprocal
     const char* raw;
     const char* hist;
     char* out;
     long long raw_row, raw_slice, hist_row, hist_slice, out_row, out_slice;
 };
 
-template <bool F16> __device__ __forceinline__ float4 ld_texel(const char* base, long long off)
-{
-    if constexpr (F16) {
-        const uint2 u = __ldg(reinterpret_cast<const uint2*>(base + off));
+// A texel as stored: 4 x binary16 or 4 x float.
+template <bool F16> struct Texel;
+template <> struct Texel<true> {
+    typedef uint2 raw;
+    static constexpr int kBytes = 8;
+    __device__ __forceinline__ static raw zero() { return make_uint2(0u, 0u); }
+    __device__ __forceinline__ static float4 value(raw u)
+    {
         const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&u.x));
         const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
         return make_float4(a.x, a.y, b.x, b.y);
-    } else {
-        return __ldg(reinterpret_cast<const float4*>(base + off));
     }
+};
+template <> struct Texel<false> {
+    typedef float4 raw;
+    static constexpr int kBytes = 16;
+    __device__ __forceinline__ static raw zero() { return make_float4(0.f, 0.f, 0.f, 0.f); }
+    __device__ __forceinline__ static float4 value(raw v) { return v; }
+};
+
+template <bool F16, class Off> __device__ __forceinline__ typename Texel<F16>::raw ld_raw(const char* base, Off off)
+{
+    return __ldg(reinterpret_cast<const typename Texel<F16>::raw*>(base + off));
 }
 
 template <bool F16> __device__ __forceinline__ void st_texel(char* base, long long off, float4 v)
@@ -77,6 +104,22 @@ __device__ __forceinline__ void mat_vec(const float* m, float x, float y, float 
     for (int r = 0; r < 4; ++r) o[r] = add(add(add(mul(m[r], x), mul(m[4 + r], y)), mul(m[8 + r], z)), mul(m[12 + r], w));
 }
 
+// x / y by the correctly rounded reciprocal r of y: one residual step is exact
+// for the box counts (every binary32 significand over 3, 6 and 9 was checked;
+// 1, 2 and 4 are exact), two steps for any divisor.  |x| < 2^100 and x / y far
+// from the subnormals, or x = 0.
+__device__ __forceinline__ float div_count(float x, float y, float r)
+{
+    const float q = mul(x, r);
+    return __fmaf_rn(__fmaf_rn(-q, y, x), r, q);
+}
+__device__ __forceinline__ float div_by(float x, float y, float r)
+{
+    const float q = div_count(x, y, r);
+    return __fmaf_rn(__fmaf_rn(-q, y, x), r, q);
+}
+constexpr float kDivMax = 1.2676506e30f;  // 2^100
+
 __device__ __forceinline__ float lerp1(float a, float b, float t) { return add(a, mul(sub(b, a), t)); }
 
 __device__ __forceinline__ float4 lerp4(float4 a, float4 b, float t)
@@ -84,132 +127,175 @@ __device__ __forceinline__ float4 lerp4(float4 a, float4 b, float t)
     return make_float4(lerp1(a.x, b.x, t), lerp1(a.y, b.y, t), lerp1(a.z, b.z, t), lerp1(a.w, b.w, t));
 }
 
-template <bool RAW16, bool OUT16>
-__global__ void __launch_bounds__(kFogTX* kFogTY) k_fog_filter(const FogArgs a)
+// Off: byte offsets within a volume (32 bits unless one is 4 GB or more).
+template <bool RAW16, bool OUT16, class Off>
+__global__ void __launch_bounds__(kFogTX* kFogRows) k_fog_filter(const FogArgs a)
 {
-    __shared__ float4 tile[kFogSH * kFogSW];
+    typedef Texel<RAW16> TR;
+    typedef Texel<OUT16> TO;
+    constexpr int kThreads = kFogTX * kFogRows;
+    constexpr int kCells = (kFogSH * kFogSW + kThreads - 1) / kThreads;
+    __shared__ float4 tile[2][kFogSH * kFogSW];
     __shared__ float view_z[kFogZC];
+    pdl_begin();
     const int x0 = blockIdx.x * kFogTX, y0 = blockIdx.y * kFogTY, z0 = blockIdx.z * kFogZC;
     const int tid = threadIdx.y * kFogTX + threadIdx.x;
-    const int x = x0 + threadIdx.x, y = y0 + threadIdx.y;
-    const bool inside = x < a.W && y < a.H;
+    const int x = x0 + threadIdx.x, yb = y0 + threadIdx.y * kFogR;
     const int nz = min(kFogZC, a.D - z0);
     const float ratio = dv(a.zfar, a.znear);
+
+    // This thread's cells of a slice's halo tile (the same in every slice), and the first slice's texels.  Cells
+    // outside the grid are staged as +0 and summed without a test: the running sum starts at +0 and so is never -0,
+    // which makes adding +0 an exact no-op, the same sums as the reference's skipped taps.
+    Off cell[kCells];
+    bool cin[kCells];
+    typename TR::raw next[kCells];
+    const char* rs = a.raw + z0 * a.raw_slice;
+#pragma unroll
+    for (int e = 0; e < kCells; ++e) {
+        const int k = tid + e * kThreads;
+        const int qy = y0 - 1 + k / kFogSW, qx = x0 - 1 + k % kFogSW;
+        cin[e] = k < kFogSH * kFogSW && qx >= 0 && qy >= 0 && qx < a.W && qy < a.H;
+        cell[e] = cin[e] ? Off(qy) * Off(a.raw_row) + Off(qx * TR::kBytes) : Off(0);
+        next[e] = cin[e] ? ld_raw<RAW16>(rs, cell[e]) : TR::zero();
+    }
 
     // Per slice of the chunk: its view depth (:74-78).
     if (tid < nz) {
         const float tz = dv(add(float(z0 + tid), 0.5f), float(a.D));
         view_z[tid] = mul(a.znear, powf(ratio, tz));
     }
-    // Per column: the normalised camera ray through the column's NDC and its cosine to the camera axis (:83-106).
-    float ray[3], rdf = 1.f, lnr = 1.f;
-    if (a.valid && inside) {
-        const float u = dv(add(float(x), 0.5f), float(a.W)), v = dv(add(float(y), 0.5f), float(a.H));
-        const float nx = sub(mul(u, 2.f), 1.f), ny = sub(1.f, mul(v, 2.f));
-        float nh[4], fh[4], fwd[3];
-        mat_vec(a.ivp, nx, ny, 0.f, 1.f, nh);
-        mat_vec(a.ivp, 0.f, 0.f, 0.f, 1.f, fh);
+    // Per column: the normalised camera ray through the column's NDC and its cosine to the camera axis (:83-106),
+    // and the in-grid members of its 3x3 box.
+    float ray[kFogR][3], rdf[kFogR], rrdf[kFogR], cnt[kFogR], rcnt[kFogR];
+    bool inside[kFogR];
+    float lnr = 1.f;
+    if (a.valid) lnr = logf(ratio);
+    const float rnear = __frcp_rn(a.znear), rlnr = __frcp_rn(lnr);
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            ray[k] = sub(dv(nh[k], nh[3]), a.cam[k]);
-            fwd[k] = sub(dv(fh[k], fh[3]), a.cam[k]);
+    for (int c = 0; c < kFogR; ++c) {
+        const int y = yb + c;
+        inside[c] = x < a.W && y < a.H;
+        rdf[c] = rrdf[c] = 1.f;
+        ray[c][0] = ray[c][1] = ray[c][2] = 0.f;
+        if (a.valid && inside[c]) {
+            const float u = dv(add(float(x), 0.5f), float(a.W)), v = dv(add(float(y), 0.5f), float(a.H));
+            const float nx = sub(mul(u, 2.f), 1.f), ny = sub(1.f, mul(v, 2.f));
+            float nh[4], fh[4], fwd[3];
+            mat_vec(a.ivp, nx, ny, 0.f, 1.f, nh);
+            mat_vec(a.ivp, 0.f, 0.f, 0.f, 1.f, fh);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                ray[c][k] = sub(dv(nh[k], nh[3]), a.cam[k]);
+                fwd[k] = sub(dv(fh[k], fh[3]), a.cam[k]);
+            }
+            const float rl = __fsqrt_rn(add(add(mul(ray[c][0], ray[c][0]), mul(ray[c][1], ray[c][1])), mul(ray[c][2], ray[c][2])));
+            const float fl = __fsqrt_rn(add(add(mul(fwd[0], fwd[0]), mul(fwd[1], fwd[1])), mul(fwd[2], fwd[2])));
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                ray[c][k] = dv(ray[c][k], rl);
+                fwd[k] = dv(fwd[k], fl);
+            }
+            const float rd = add(add(mul(ray[c][0], fwd[0]), mul(ray[c][1], fwd[1])), mul(ray[c][2], fwd[2]));
+            rdf[c] = rd > 1e-4f ? rd : 1e-4f;
+            rrdf[c] = __frcp_rn(rdf[c]);
         }
-        const float rl = __fsqrt_rn(add(add(mul(ray[0], ray[0]), mul(ray[1], ray[1])), mul(ray[2], ray[2])));
-        const float fl = __fsqrt_rn(add(add(mul(fwd[0], fwd[0]), mul(fwd[1], fwd[1])), mul(fwd[2], fwd[2])));
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            ray[k] = dv(ray[k], rl);
-            fwd[k] = dv(fwd[k], fl);
-        }
-        rdf = add(add(mul(ray[0], fwd[0]), mul(ray[1], fwd[1])), mul(ray[2], fwd[2]));
-        rdf = rdf > 1e-4f ? rdf : 1e-4f;
-        lnr = logf(ratio);
-    }
-    // In-grid members of the column's 3x3 box.
-    float n = 0.f;
-#pragma unroll
-    for (int dy = -1; dy <= 1; ++dy)
-#pragma unroll
-        for (int dx = -1; dx <= 1; ++dx)
-            if (x + dx >= 0 && x + dx <= a.W - 1 && y + dy >= 0 && y + dy <= a.H - 1) n = add(n, 1.f);
-    const float cnt = fmaxf(n, 1.f);
-
-    for (int zi = 0; zi < nz; ++zi) {
-        const int z = z0 + zi;
-        const char* rs = a.raw + z * a.raw_slice;
-        __syncthreads();  // the previous slice's tile is consumed (and view_z is written before the first use)
-        for (int k = tid; k < kFogSH * kFogSW; k += kFogTX * kFogTY) {
-            const int qy = y0 - 1 + k / kFogSW, qx = x0 - 1 + k % kFogSW;
-            float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (qx >= 0 && qy >= 0 && qx < a.W && qy < a.H) q = ld_texel<RAW16>(rs, qy * a.raw_row + qx * (RAW16 ? 8LL : 16LL));
-            tile[k] = q;
-        }
-        __syncthreads();
-        if (!inside) continue;
-
-        // 1. 3x3 mean over the in-grid neighbours of the slice (:152-166).  Cells outside the grid are staged
-        // as +0 and summed without a test: the running sum starts at +0 and so is never -0, which makes adding
-        // +0 an exact no-op, the same sums as the reference's skipped taps.
-        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+        float n = 0.f;
 #pragma unroll
         for (int dy = -1; dy <= 1; ++dy)
 #pragma unroll
-            for (int dx = -1; dx <= 1; ++dx) {
-                const float4 q = tile[(threadIdx.y + 1 + dy) * kFogSW + threadIdx.x + 1 + dx];
-                s = make_float4(add(s.x, q.x), add(s.y, q.y), add(s.z, q.z), add(s.w, q.w));
+            for (int dx = -1; dx <= 1; ++dx)
+                if (x + dx >= 0 && x + dx <= a.W - 1 && y + dy >= 0 && y + dy <= a.H - 1) n = add(n, 1.f);
+        cnt[c] = fmaxf(n, 1.f);
+        rcnt[c] = __frcp_rn(cnt[c]);
+    }
+
+    for (int zi = 0; zi < nz; ++zi) {
+        const int z = z0 + zi;
+        float4* t = tile[zi & 1];
+#pragma unroll
+        for (int e = 0; e < kCells; ++e)
+            if (tid + e * kThreads < kFogSH * kFogSW) t[tid + e * kThreads] = TR::value(next[e]);
+        // One barrier per slice: a thread reaches the next slice's stores into this half of the tile only after the
+        // next barrier, which every thread passes after it has read this slice.
+        __syncthreads();
+        if (zi + 1 < nz) {
+            rs += a.raw_slice;
+#pragma unroll
+            for (int e = 0; e < kCells; ++e) next[e] = cin[e] ? ld_raw<RAW16>(rs, cell[e]) : TR::zero();
+        }
+
+        // 1. 3x3 mean over the in-grid neighbours of the slice (:152-166), summed in the reference's order
+        float4 s[kFogR];
+#pragma unroll
+        for (int c = 0; c < kFogR; ++c) s[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int r = 0; r < kFogR + 2; ++r)
+#pragma unroll
+            for (int dx = 0; dx < 3; ++dx) {
+                const float4 q = t[(threadIdx.y * kFogR + r) * kFogSW + threadIdx.x + dx];
+#pragma unroll
+                for (int c = 0; c < kFogR; ++c)
+                    if (r >= c && r <= c + 2) s[c] = make_float4(add(s[c].x, q.x), add(s[c].y, q.y), add(s[c].z, q.z), add(s[c].w, q.w));
             }
-        const float4 sp = make_float4(dv(s.x, cnt), dv(s.y, cnt), dv(s.z, cnt), dv(s.w, cnt));
-        char* op = a.out + z * a.out_slice + y * a.out_row + x * (OUT16 ? 8LL : 16LL);
-        if (!a.valid) {
-            st_texel<OUT16>(op, 0, sp);
-            continue;
-        }
 
-        // 2. froxel centre on the column's ray at the slice's view depth (:100-106)
-        const float t = dv(view_z[zi], rdf);
-        const float wx = add(a.cam[0], mul(ray[0], t)), wy = add(a.cam[1], mul(ray[1], t)),
-                    wz = add(a.cam[2], mul(ray[2], t));
+#pragma unroll
+        for (int c = 0; c < kFogR; ++c) {
+            if (!inside[c]) continue;
+            float4 sp;
+            if (fmaxf(fmaxf(fabsf(s[c].x), fabsf(s[c].y)), fmaxf(fabsf(s[c].z), fabsf(s[c].w))) < kDivMax)
+                sp = make_float4(div_count(s[c].x, cnt[c], rcnt[c]), div_count(s[c].y, cnt[c], rcnt[c]),
+                                 div_count(s[c].z, cnt[c], rcnt[c]), div_count(s[c].w, cnt[c], rcnt[c]));
+            else
+                sp = make_float4(dv(s[c].x, cnt[c]), dv(s[c].y, cnt[c]), dv(s[c].z, cnt[c]), dv(s[c].w, cnt[c]));
+            float4 res = sp;
+            if (a.valid) {
+                // 2. froxel centre on the column's ray at the slice's view depth (:100-106)
+                const float tt = a.plain_div ? dv(view_z[zi], rdf[c]) : div_by(view_z[zi], rdf[c], rrdf[c]);
+                const float wx = add(a.cam[0], mul(ray[c][0], tt)), wy = add(a.cam[1], mul(ray[c][1], tt)),
+                            wz = add(a.cam[2], mul(ray[c][2], tt));
 
-        // 3. previous-frame froxel coordinates and rejections (:177-213)
-        float pc[4];
-        mat_vec(a.pvp, wx, wy, wz, 1.f, pc);
-        if (pc[3] <= 1e-4f) {
-            st_texel<OUT16>(op, 0, sp);
-            continue;
+                // 3. previous-frame froxel coordinates and rejections (:177-213)
+                float pc[4];
+                mat_vec(a.pvp, wx, wy, wz, 1.f, pc);
+                const float pz = pc[3];
+                float ndx, ndy, lt;
+                if (!a.plain_div && fmaxf(fmaxf(fabsf(pc[0]), fabsf(pc[1])), fabsf(pz)) < kDivMax) {
+                    const float rw = __frcp_rn(pz);
+                    ndx = div_by(pc[0], pz, rw);
+                    ndy = div_by(pc[1], pz, rw);
+                    lt = div_by(logf(div_by(pz, a.znear, rnear)), lnr, rlnr);
+                } else {
+                    ndx = dv(pc[0], pz);
+                    ndy = dv(pc[1], pz);
+                    lt = dv(logf(dv(pz, a.znear)), lnr);
+                }
+                const float fx = mul(add(mul(ndx, 0.5f), 0.5f), float(a.W));
+                const float fy = mul(add(mul(-ndy, 0.5f), 0.5f), float(a.H));
+                const float fz = sub(mul(lt, float(a.D)), 0.5f);
+                const bool rej = pz <= 1e-4f || pz < a.znear || pz > a.zfar || fx < 0.f || fx >= float(a.W) || fy < 0.f ||
+                                 fy >= float(a.H) || fz < 0.f || fz >= float(a.D);
+                if (!rej) {
+                    // 4. trilinear history, clamp-to-edge (:111-140), then the EMA (:216-225)
+                    const int ix = int(floorf(fx)), iy = int(floorf(fy)), iz = int(floorf(fz));
+                    const float ax = sub(fx, float(ix)), ay = sub(fy, float(iy)), az = sub(fz, float(iz));
+                    const int xa = min(max(ix, 0), a.W - 1), xb = min(max(ix + 1, 0), a.W - 1);
+                    const int ya = min(max(iy, 0), a.H - 1), yc = min(max(iy + 1, 0), a.H - 1);
+                    const int za = min(max(iz, 0), a.D - 1), zb = min(max(iz + 1, 0), a.D - 1);
+                    const Off oxa = Off(xa * TO::kBytes), oxb = Off(xb * TO::kBytes);
+                    const Off ra = Off(za) * Off(a.hist_slice) + Off(ya) * Off(a.hist_row);
+                    const Off dy = Off(yc - ya) * Off(a.hist_row), dz = Off(zb - za) * Off(a.hist_slice);
+                    typename TO::raw h[8];
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                        h[k] = ld_raw<OUT16>(a.hist, ra + (k & 4 ? dz : Off(0)) + (k & 2 ? dy : Off(0)) + (k & 1 ? oxb : oxa));
+                    const float4 c0 = lerp4(lerp4(TO::value(h[0]), TO::value(h[1]), ax), lerp4(TO::value(h[2]), TO::value(h[3]), ax), ay);
+                    const float4 c1 = lerp4(lerp4(TO::value(h[4]), TO::value(h[5]), ax), lerp4(TO::value(h[6]), TO::value(h[7]), ax), ay);
+                    res = lerp4(lerp4(c0, c1, az), sp, a.alpha);
+                }
+            }
+            st_texel<OUT16>(a.out, z * a.out_slice + (yb + c) * a.out_row + x * (long long)TO::kBytes, res);
         }
-        const float ndx = dv(pc[0], pc[3]), ndy = dv(pc[1], pc[3]);
-        const float fx = mul(add(mul(ndx, 0.5f), 0.5f), float(a.W));
-        const float fy = mul(add(mul(-ndy, 0.5f), 0.5f), float(a.H));
-        const float pz = pc[3];
-        if (pz < a.znear || pz > a.zfar) {
-            st_texel<OUT16>(op, 0, sp);
-            continue;
-        }
-        const float lt = dv(logf(dv(pz, a.znear)), lnr);
-        const float fz = sub(mul(lt, float(a.D)), 0.5f);
-        if (fx < 0.f || fx >= float(a.W) || fy < 0.f || fy >= float(a.H) || fz < 0.f || fz >= float(a.D)) {
-            st_texel<OUT16>(op, 0, sp);
-            continue;
-        }
-
-        // 4. trilinear history, clamp-to-edge (:111-140), then the EMA (:216-225)
-        const int ix = int(floorf(fx)), iy = int(floorf(fy)), iz = int(floorf(fz));
-        const float ax = sub(fx, float(ix)), ay = sub(fy, float(iy)), az = sub(fz, float(iz));
-        const int xa = min(max(ix, 0), a.W - 1), xb = min(max(ix + 1, 0), a.W - 1);
-        const int ya = min(max(iy, 0), a.H - 1), yb = min(max(iy + 1, 0), a.H - 1);
-        const int za = min(max(iz, 0), a.D - 1), zb = min(max(iz + 1, 0), a.D - 1);
-        const long long tb = OUT16 ? 8LL : 16LL;
-        const long long oxa = xa * tb, oxb = xb * tb, oya = ya * a.hist_row, oyb = yb * a.hist_row;
-        const char* ha = a.hist + za * a.hist_slice;
-        const char* hb = a.hist + zb * a.hist_slice;
-        const float4 c000 = ld_texel<OUT16>(ha, oya + oxa), c100 = ld_texel<OUT16>(ha, oya + oxb);
-        const float4 c010 = ld_texel<OUT16>(ha, oyb + oxa), c110 = ld_texel<OUT16>(ha, oyb + oxb);
-        const float4 c001 = ld_texel<OUT16>(hb, oya + oxa), c101 = ld_texel<OUT16>(hb, oya + oxb);
-        const float4 c011 = ld_texel<OUT16>(hb, oyb + oxa), c111 = ld_texel<OUT16>(hb, oyb + oxb);
-        const float4 c0 = lerp4(lerp4(c000, c100, ax), lerp4(c010, c110, ax), ay);
-        const float4 c1 = lerp4(lerp4(c001, c101, ax), lerp4(c011, c111, ax), ay);
-        const float4 h = lerp4(c0, c1, az);
-        st_texel<OUT16>(op, 0, lerp4(h, sp, a.alpha));
     }
 }
 
@@ -251,8 +337,8 @@ int tg_fog_filter(const tg_fog_filter_params* p, const tg_volume* raw, const tg_
 {
     if (!p) return fail(TG_ERR_INVALID, "null parameters");
     const uint32_t W = p->froxel_width, H = p->froxel_height, D = p->froxel_depth;
-    if (W == 0 || H == 0 || D == 0 || W > 65535u * kFogTX || H > 65535u * kFogTY || D > 65535u)
-        return fail(TG_ERR_INVALID, "froxel grid %ux%ux%u outside 1..(2097120, 524280, 65535)", W, H, D);
+    if (W == 0 || H == 0 || D == 0 || W > 65535u * kFogTX || H > 65535u * kFogRows || D > 65535u)
+        return fail(TG_ERR_INVALID, "froxel grid %ux%ux%u outside 1..(2097120, 262140, 65535)", W, H, D);
     if (!(p->near_plane > 0.f) || !(p->far_plane > p->near_plane))
         return fail(TG_ERR_INVALID, "depth range needs 0 < near_plane < far_plane");
     VolGeom gr, gh, go;
@@ -276,6 +362,8 @@ int tg_fog_filter(const tg_fog_filter_params* p, const tg_volume* raw, const tg_
     a.H = int(H);
     a.D = int(D);
     a.valid = p->history_valid != 0;
+    // quotients by reciprocal stay far from overflow and the subnormals while the depth range is within these bounds
+    a.plain_div = !(p->near_plane >= 1e-15f && p->far_plane <= 1e15f && p->far_plane / p->near_plane >= 1.0001f);
     a.raw = static_cast<const char*>(raw->ptr);
     a.hist = static_cast<const char*>(hist->ptr);
     a.out = static_cast<char*>(out->ptr);
@@ -286,18 +374,17 @@ int tg_fog_filter(const tg_fog_filter_params* p, const tg_volume* raw, const tg_
     a.out_row = go.row;
     a.out_slice = go.slice;
     const dim3 grid((W + kFogTX - 1) / kFogTX, (H + kFogTY - 1) / kFogTY, (D + kFogZC - 1) / kFogZC),
-        block(kFogTX, kFogTY);
+        block(kFogTX, kFogRows);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const bool r16 = raw->format == TG_FMT_RGBA16F, o16 = out->format == TG_FMT_RGBA16F;
-    if (r16 && o16)
-        k_fog_filter<true, true><<<grid, block, 0, s>>>(a);
-    else if (r16)
-        k_fog_filter<true, false><<<grid, block, 0, s>>>(a);
-    else if (o16)
-        k_fog_filter<false, true><<<grid, block, 0, s>>>(a);
-    else
-        k_fog_filter<false, false><<<grid, block, 0, s>>>(a);
-    const cudaError_t e = cudaGetLastError();
+    const bool wide = gr.bytes > 0xffffffffLL || gh.bytes > 0xffffffffLL;
+    typedef void (*Fn)(const FogArgs);
+    static const Fn fns[2][4] = {
+        {k_fog_filter<false, false, uint32_t>, k_fog_filter<false, true, uint32_t>, k_fog_filter<true, false, uint32_t>,
+         k_fog_filter<true, true, uint32_t>},
+        {k_fog_filter<false, false, uint64_t>, k_fog_filter<false, true, uint64_t>, k_fog_filter<true, false, uint64_t>,
+         k_fog_filter<true, true, uint64_t>}};
+    const cudaError_t e = launch_chain(fns[wide][2 * r16 + o16], grid, block, s, a);
     if (e != cudaSuccess) return fail(TG_ERR_CUDA, "fog filter launch failed: %s", cudaGetErrorString(e));
     return TG_OK;
 }
