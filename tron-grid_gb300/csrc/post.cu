@@ -11,8 +11,19 @@
 //
 // All arithmetic is explicitly rounded IEEE single precision in the shaders'
 // order (sums left to right, no contraction into FMA); only the sRGB curve's
-// power (exp2f / log2f) is CUDA's.  One thread per output texel, 32 x 8
-// threads per CTA.
+// power (exp2f / log2f) is CUDA's.  Quotients by a divisor that several of them
+// share are formed from its correctly rounded reciprocal and FMA residuals, which
+// rounds correctly while nothing overflows (Markstein 1990; Brisebarre, Muller
+// and Raina 2004).
+//
+// What bounds it: FP32 issue in the extraction and the post pass (the 4K chain's
+// compulsory 100 MB take 15 us of the 6.8 TB/s a copy reaches), launch latency in
+// the small upsamples.  So work that neighbours share is done once: an upsample
+// thread owns the 2x2 texels that share a tent, a post thread two pixels that
+// share a bloom texel (and, away from the corners, all three samples of a pixel
+// are one), and the launches overlap by programmatic dependent launch.  Measured:
+// the 3840x2160 chain (rgba16f to BGRA8) 166 -> 115 us, 1281x721 (rgba32f to
+// rgba32f) 49.8 -> 26.1 us.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -21,6 +32,7 @@
 #include <cstdint>
 #include <new>
 
+#include "svgf_device.cuh"
 #include "svgf_internal.h"
 #include "tg_post.h"
 
@@ -34,6 +46,16 @@ __device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b);
 __device__ __forceinline__ float sub(float a, float b) { return __fsub_rn(a, b); }
 __device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ float dv(float a, float b) { return __fdiv_rn(a, b); }
+
+// x / y by the correctly rounded reciprocal r of y, |x| < 2^100 and x / y far
+// from the subnormals (or too small to matter to the caller), or x = 0.
+__device__ __forceinline__ float div_by(float x, float y, float r)
+{
+    float q = mul(x, r);
+    q = __fmaf_rn(__fmaf_rn(-q, y, x), r, q);
+    return __fmaf_rn(__fmaf_rn(-q, y, x), r, q);
+}
+constexpr float kDivMax = 1.2676506e30f;  // 2^100
 
 struct C3 {
     float r, g, b;
@@ -76,26 +98,48 @@ __device__ __forceinline__ C3 round16(C3 c)
     return {__half2float(__float2half_rn(c.r)), __half2float(__float2half_rn(c.g)), __half2float(__float2half_rn(c.b))};
 }
 
-// Mip-0 texel (x, y) of the extraction (bloomExtractMain), before the fp16 store.
-template <bool HDR16> __device__ __forceinline__ C3 extract_texel(const char* hdr, long long pitch, int W, int H, int x, int y, float thr)
+// Two horizontally adjacent HDR pixels (x even) of row y: one 16-byte load of
+// binary16 texels where the image is aligned for it (`vec`).
+template <bool F16> __device__ __forceinline__ void ld_hdr2(const char* base, long long pitch, int x, int x1, int y, bool vec, C3 (&c)[2])
+{
+    if (F16 && vec) {
+        const uint4 u = *reinterpret_cast<const uint4*>(base + y * pitch + x * 8LL);
+        const float2 a0 = __half22float2(*reinterpret_cast<const __half2*>(&u.x)), a1 = __half22float2(*reinterpret_cast<const __half2*>(&u.z));
+        c[0] = {a0.x, a0.y, __half2float(__ushort_as_half((unsigned short)(u.y & 0xffffu)))};
+        c[1] = {a1.x, a1.y, __half2float(__ushort_as_half((unsigned short)(u.w & 0xffffu)))};
+    } else {
+        c[0] = ld_hdr<F16>(base, pitch, x, y);
+        c[1] = ld_hdr<F16>(base, pitch, x1, y);
+    }
+}
+
+// Mip-0 texel of the extraction (bloomExtractMain) from its 2x2 HDR block, before the fp16 store.  A sample below
+// the threshold is zero: its luminance is 0 and its weight 1.  (No sample is infinite and below the threshold, so
+// selecting equals the shader's multiplication by 0 or 1.)
+__device__ __forceinline__ C3 extract_texel(const C3 (&in)[4], float thr)
 {
     C3 s[4];
     float w[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        C3 c = ld_hdr<HDR16>(hdr, pitch, min(2 * x + (k & 1), W - 1), min(2 * y + (k >> 1), H - 1));
+        C3 c = in[k];
         c = {c.r > 0.f ? c.r : 0.f, c.g > 0.f ? c.g : 0.f, c.b > 0.f ? c.b : 0.f};
-        const float keep = lum(c) >= thr ? 1.f : 0.f;
-        c = {mul(c.r, keep), mul(c.g, keep), mul(c.b, keep)};
-        s[k] = c;
-        w[k] = dv(1.f, add(1.f, lum(c)));
+        const float l = lum(c);
+        const bool keep = l >= thr;
+        s[k] = keep ? c : C3{0.f, 0.f, 0.f};
+        w[k] = keep ? __frcp_rn(add(1.f, l)) : 1.f;
     }
     const float ws = add(add(add(w[0], w[1]), w[2]), w[3]);
     const float den = ws > 1e-7f ? ws : 1e-7f;
-    auto acc = [&](float C3::*m) {
-        return dv(add(add(add(mul(s[0].*m, w[0]), mul(s[1].*m, w[1])), mul(s[2].*m, w[2])), mul(s[3].*m, w[3])), den);
+    auto num = [&](float C3::*m) {
+        return add(add(add(mul(s[0].*m, w[0]), mul(s[1].*m, w[1])), mul(s[2].*m, w[2])), mul(s[3].*m, w[3]));
     };
-    return {acc(&C3::r), acc(&C3::g), acc(&C3::b)};
+    const C3 n = {num(&C3::r), num(&C3::g), num(&C3::b)};
+    if (fmaxf(fmaxf(n.r, n.g), n.b) < kDivMax) {  // (a quotient too small for div_by rounds to a binary16 zero)
+        const float rd = __frcp_rn(den);
+        return {div_by(n.r, den, rd), div_by(n.g, den, rd), div_by(n.b, den, rd)};
+    }
+    return {dv(n.r, den), dv(n.g, den), dv(n.b, den)};
 }
 
 // Mip i of the box-downsample chain from the 2x2 block of mip i-1 (bloomDownsampleMain).
@@ -118,16 +162,34 @@ struct MipSet {
 };
 
 template <bool HDR16>
-__global__ void __launch_bounds__(256) k_bloom_pyramid(const char* hdr, long long pitch, int W, int H, MipSet ms, float thr)
+__global__ void __launch_bounds__(256) k_bloom_pyramid(const char* hdr, long long pitch, int W, int H, MipSet ms, float thr, int vec)
 {
     __shared__ float sa[3][kPyrT * kPyrT];  // ping-pong tiles of one mip level, one plane per channel
     __shared__ float sb[3][kPyrT * kPyrT];
     const int tid = threadIdx.x;
     const int X0 = blockIdx.x * kPyrT, Y0 = blockIdx.y * kPyrT;
-    for (int k = tid; k < kPyrT * kPyrT; k += 256) {
+    pdl_begin();
+    // every HDR load of the thread's four texels is issued before the first is used
+    constexpr int kPer = kPyrT * kPyrT / 256;
+    C3 in[kPer][4];
+#pragma unroll
+    for (int e = 0; e < kPer; ++e) {
+        const int k = tid + e * 256;
+        const int x = min(X0 + k % kPyrT, ms.m[0].w - 1), y = min(Y0 + k / kPyrT, ms.m[0].h - 1);
+        C3 row[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            ld_hdr2<HDR16>(hdr, pitch, min(2 * x, W - 1), min(2 * x + 1, W - 1), min(2 * y + j, H - 1), vec, row);
+            in[e][2 * j] = row[0];
+            in[e][2 * j + 1] = row[1];
+        }
+    }
+#pragma unroll
+    for (int e = 0; e < kPer; ++e) {
+        const int k = tid + e * 256;
         const int x = X0 + k % kPyrT, y = Y0 + k / kPyrT;
         if (x >= ms.m[0].w || y >= ms.m[0].h) continue;
-        const C3 c = round16(extract_texel<HDR16>(hdr, pitch, W, H, x, y, thr));
+        const C3 c = round16(extract_texel(in[e], thr));
         st_h4(ms.m[0].p, (long long)y * ms.m[0].w + x, c);
         sa[0][k] = c.r;
         sa[1][k] = c.g;
@@ -164,6 +226,7 @@ __global__ void __launch_bounds__(256) k_bloom_pyramid(const char* hdr, long lon
 
 __global__ void __launch_bounds__(kPostTX* kPostTY) k_bloom_down(Mip s, Mip d)
 {
+    pdl_begin();
     const int x = blockIdx.x * kPostTX + threadIdx.x, y = blockIdx.y * kPostTY + threadIdx.y;
     if (x >= d.w || y >= d.h) return;
     C3 c[4];
@@ -173,11 +236,23 @@ __global__ void __launch_bounds__(kPostTX* kPostTY) k_bloom_down(Mip s, Mip d)
     st_h4(d.p, (long long)y * d.w + x, box4(c));
 }
 
+// One thread per 2x2 block of texels: the four add the same tent of the next mip
+// (around x / 2, y / 2).
 __global__ void __launch_bounds__(kPostTX* kPostTY) k_bloom_up(Mip s, Mip d)
 {
-    const int x = blockIdx.x * kPostTX + threadIdx.x, y = blockIdx.y * kPostTY + threadIdx.y;
-    if (x >= d.w || y >= d.h) return;
-    const int bx = x / 2, by = y / 2;
+    pdl_begin();
+    const int bx = blockIdx.x * kPostTX + threadIdx.x, by = blockIdx.y * kPostTY + threadIdx.y;
+    if (2 * bx >= d.w || 2 * by >= d.h) return;
+    uint2* o[4];
+    C3 e[4];
+    bool in[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int x = 2 * bx + (k & 1), y = 2 * by + (k >> 1);
+        in[k] = x < d.w && y < d.h;
+        o[k] = d.p + (long long)y * d.w + x;
+        e[k] = in[k] ? ld_h4(o[k], 0) : C3{0.f, 0.f, 0.f};
+    }
     C3 sum = {0.f, 0.f, 0.f};
 #pragma unroll
     for (int dy = -1; dy <= 1; ++dy)
@@ -187,12 +262,13 @@ __global__ void __launch_bounds__(kPostTX* kPostTY) k_bloom_up(Mip s, Mip d)
             const C3 c = ld_h4(s.p, (long long)min(max(by + dy, 0), s.h - 1) * s.w + min(max(bx + dx, 0), s.w - 1));
             sum = {add(sum.r, mul(wk, c.r)), add(sum.g, mul(wk, c.g)), add(sum.b, mul(wk, c.b))};
         }
-    const long long i = (long long)y * d.w + x;
-    const C3 e = ld_h4(d.p, i);
-    st_h4(d.p, i, {add(e.r, sum.r), add(e.g, sum.g), add(e.b, sum.b)});
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        if (in[k]) st_h4(o[k], 0, {add(e[k].r, sum.r), add(e[k].g, sum.g), add(e[k].b, sum.b)});
 }
 
-__device__ __forceinline__ float sat(float v) { return v < 0.f ? 0.f : (v > 1.f ? 1.f : v); }
+// Clamp to [0, 1].  (The shader's clamp keeps a NaN, which the sRGB curve then maps to 0; here it is 0 at once.)
+__device__ __forceinline__ float sat(float v) { return __saturatef(v); }
 
 // c^(1/2.4) for c in (0.0031308, 1] as exp2f(log2f(c) / 2.4): full-precision library calls (a few ulp),
 // far cheaper than the general powf; the 8-bit output absorbs the difference almost everywhere.
@@ -222,27 +298,9 @@ __constant__ float kAcesOut[9] = {1.60475f, -0.53108f, -0.07367f, -0.10208f, 1.1
 
 enum OutFmt { OUT_BGRA8 = 0, OUT_RGBA8 = 1, OUT_RGBA32F = 2 };
 
-template <bool HDR16, int OUT>
-__global__ void __launch_bounds__(kPostTX* kPostTY)
-    k_post(const char* hdr, long long hpitch, char* out, long long opitch, int W, int H, Mip bl, float strength)
+// ACES, sRGB, grade and vignette of one lit pixel.
+__device__ __forceinline__ C3 display(C3 c, float d2)
 {
-    const int x = blockIdx.x * kPostTX + threadIdx.x, y = blockIdx.y * kPostTY + threadIdx.y;
-    if (x >= W || y >= H) return;
-    const float u = dv(add(float(x), 0.5f), float(W)), v = dv(add(float(y), 0.5f), float(H));
-    const float ox = sub(u, 0.5f), oy = sub(v, 0.5f);
-    const float d2 = add(mul(ox, ox), mul(oy, oy));
-    const int px = int(mul(mul(mul(ox, d2), 0.0015f), float(W))), py = int(mul(mul(mul(oy, d2), 0.0015f), float(H)));
-    auto sample = [&](int cx, int cy) {
-        cx = min(cx, W - 1);
-        cy = min(cy, H - 1);
-        const C3 h = ld_hdr<HDR16>(hdr, hpitch, cx, cy);
-        const C3 b = ld_h4(bl.p, (long long)min(cy / 2, bl.h - 1) * bl.w + min(cx / 2, bl.w - 1));
-        return C3{add(h.r, mul(strength, b.r)), add(h.g, mul(strength, b.g)), add(h.b, mul(strength, b.b))};
-    };
-    C3 c;
-    c.r = sample(min(max(x + px, 0), W - 1), min(max(y + py, 0), H - 1)).r;
-    c.g = sample(x, y).g;
-    c.b = sample(min(max(x - px, 0), W - 1), min(max(y - py, 0), H - 1)).b;
     c = mat3(kAcesIn, c);
     c = {fit(c.r), fit(c.g), fit(c.b)};
     c = mat3(kAcesOut, c);
@@ -250,16 +308,67 @@ __global__ void __launch_bounds__(kPostTX* kPostTY)
     const float l = lum(c);
     const C3 cool = {mul(l, 0.9f), mul(l, 0.95f), mul(l, 1.1f)};
     c = {add(c.r, mul(sub(cool.r, c.r), 0.15f)), add(c.g, mul(sub(cool.g, c.g), 0.15f)), add(c.b, mul(sub(cool.b, c.b), 0.15f))};
-    const float vig = sat(sub(1.f, mul(add(mul(ox, ox), mul(oy, oy)), 1.5f)));
-    c = {mul(c.r, vig), mul(c.g, vig), mul(c.b, vig)};
+    const float vig = sat(sub(1.f, mul(d2, 1.5f)));
+    return {mul(c.r, vig), mul(c.g, vig), mul(c.b, vig)};
+}
+
+// Two pixels (2t, 2t + 1) of a row per thread; they share a bloom texel.  vec:
+// the images are aligned for 16-byte HDR loads (binary16) and for paired stores.
+// rw, rh: the reciprocals of W and H.
+template <bool HDR16, int OUT>
+__global__ void __launch_bounds__(kPostTX* kPostTY)
+    k_post(const char* hdr, long long hpitch, char* out, long long opitch, int W, int H, Mip bl, float strength, float rw,
+           float rh, int vec)
+{
+    pdl_begin();
+    const int x = 2 * (blockIdx.x * kPostTX + threadIdx.x), y = blockIdx.y * kPostTY + threadIdx.y;
+    if (x >= W || y >= H) return;
+    const bool two = x + 1 < W;
+    C3 h[2];
+    ld_hdr2<HDR16>(hdr, hpitch, x, two ? x + 1 : x, y, (vec & 1) && two, h);
+    const C3 b = ld_h4(bl.p, (long long)min(y / 2, bl.h - 1) * bl.w + min(x / 2, bl.w - 1));
+    const C3 sb = {mul(strength, b.r), mul(strength, b.g), mul(strength, b.b)};
+    const float v = div_by(add(float(y), 0.5f), float(H), rh), oy = sub(v, 0.5f), oy2 = mul(oy, oy);
+    C3 res[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const float u = div_by(add(float(x + k), 0.5f), float(W), rw), ox = sub(u, 0.5f);
+        const float d2 = add(mul(ox, ox), oy2);
+        const int px = int(mul(mul(mul(ox, d2), 0.0015f), float(W))), py = int(mul(mul(mul(oy, d2), 0.0015f), float(H)));
+        C3 c = {add(h[k].r, sb.r), add(h[k].g, sb.g), add(h[k].b, sb.b)};
+        if (px != 0 || py != 0) {  // chromatic aberration of a pixel or more: only towards the corners
+            auto sample = [&](int cx, int cy) {
+                cx = min(max(cx, 0), W - 1);
+                cy = min(max(cy, 0), H - 1);
+                const C3 hs = ld_hdr<HDR16>(hdr, hpitch, cx, cy);
+                const C3 bs = ld_h4(bl.p, (long long)min(cy / 2, bl.h - 1) * bl.w + min(cx / 2, bl.w - 1));
+                return C3{add(hs.r, mul(strength, bs.r)), add(hs.g, mul(strength, bs.g)), add(hs.b, mul(strength, bs.b))};
+            };
+            c.r = sample(x + k + px, y + py).r;
+            c.b = sample(x + k - px, y - py).b;
+        }
+        res[k] = display(c, d2);
+    }
     char* row = out + y * opitch;
     if constexpr (OUT == OUT_RGBA32F) {
-        reinterpret_cast<float4*>(row)[x] = make_float4(c.r, c.g, c.b, 1.f);
+        float4* o = reinterpret_cast<float4*>(row) + x;
+        o[0] = make_float4(res[0].r, res[0].g, res[0].b, 1.f);
+        if (two) o[1] = make_float4(res[1].r, res[1].g, res[1].b, 1.f);
     } else {
-        auto q = [](float f) { return __float2uint_rn(__fmul_rn(sat(f), 255.0f)); };
-        const uint32_t r = q(c.r), g = q(c.g), b = q(c.b);
-        reinterpret_cast<uint32_t*>(row)[x] = OUT == OUT_BGRA8 ? (b | (g << 8) | (r << 16) | (255u << 24))
-                                                                : (r | (g << 8) | (b << 16) | (255u << 24));
+        uint32_t px8[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            auto q = [](float f) { return __float2uint_rn(__fmul_rn(sat(f), 255.0f)); };
+            const uint32_t r = q(res[k].r), g = q(res[k].g), bb = q(res[k].b);
+            px8[k] = OUT == OUT_BGRA8 ? (bb | (g << 8) | (r << 16) | (255u << 24)) : (r | (g << 8) | (bb << 16) | (255u << 24));
+        }
+        uint32_t* o = reinterpret_cast<uint32_t*>(row) + x;
+        if (two && (vec & 2)) {
+            *reinterpret_cast<uint2*>(o) = make_uint2(px8[0], px8[1]);
+        } else {
+            o[0] = px8[0];
+            if (two) o[1] = px8[1];
+        }
     }
 }
 
@@ -383,29 +492,27 @@ int tg_post_process(tg_post* s, const tg_image* hdr, const tg_image* out, void* 
     const char* hb = static_cast<const char*>(hdr->ptr);
     const bool h16 = hdr->format == TG_FMT_RGBA16F;
     const int W = int(s->w), H = int(s->h);
+    // bit 0: pairs of binary16 HDR texels start on 16 bytes; bit 1: pairs of 4-byte display texels on 8
+    const int vec = (reinterpret_cast<uintptr_t>(hb) % 16 == 0 && hp % 16 == 0 && W > 1 ? 1 : 0) |
+                    (reinterpret_cast<uintptr_t>(out->ptr) % 8 == 0 && op % 8 == 0 ? 2 : 0);
     // extraction + mips 1..5 in one launch; mips beyond the sixth (max_mips > 6) one launch each
     MipSet ms;
     ms.n = std::min(s->n, kPyrLevels);
     for (int i = 0; i < ms.n; ++i) ms.m[i] = s->mip[i];
     const dim3 pgrid((s->mip[0].w + kPyrT - 1) / kPyrT, (s->mip[0].h + kPyrT - 1) / kPyrT);
-    if (h16)
-        k_bloom_pyramid<true><<<pgrid, 256, 0, cs>>>(hb, hp, W, H, ms, s->p.bloom_threshold);
-    else
-        k_bloom_pyramid<false><<<pgrid, 256, 0, cs>>>(hb, hp, W, H, ms, s->p.bloom_threshold);
-    for (int i = kPyrLevels; i < s->n; ++i) k_bloom_down<<<grid(s->mip[i].w, s->mip[i].h), blk, 0, cs>>>(s->mip[i - 1], s->mip[i]);
-    for (int i = s->n - 2; i >= 0; --i) k_bloom_up<<<grid(s->mip[i].w, s->mip[i].h), blk, 0, cs>>>(s->mip[i + 1], s->mip[i]);
-    char* ob = static_cast<char*>(out->ptr);
-    const float str = s->p.bloom_strength;
-    const dim3 pg = grid(W, H);
-    switch ((h16 ? 10 : 0) + (out->format == TG_FMT_BGRA8 ? 0 : out->format == TG_FMT_RGBA8 ? 1 : 2)) {
-    case 10: k_post<true, OUT_BGRA8><<<pg, blk, 0, cs>>>(hb, hp, ob, op, W, H, s->mip[0], str); break;
-    case 11: k_post<true, OUT_RGBA8><<<pg, blk, 0, cs>>>(hb, hp, ob, op, W, H, s->mip[0], str); break;
-    case 12: k_post<true, OUT_RGBA32F><<<pg, blk, 0, cs>>>(hb, hp, ob, op, W, H, s->mip[0], str); break;
-    case 0: k_post<false, OUT_BGRA8><<<pg, blk, 0, cs>>>(hb, hp, ob, op, W, H, s->mip[0], str); break;
-    case 1: k_post<false, OUT_RGBA8><<<pg, blk, 0, cs>>>(hb, hp, ob, op, W, H, s->mip[0], str); break;
-    default: k_post<false, OUT_RGBA32F><<<pg, blk, 0, cs>>>(hb, hp, ob, op, W, H, s->mip[0], str); break;
-    }
-    const cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_chain(h16 ? k_bloom_pyramid<true> : k_bloom_pyramid<false>, pgrid, dim3(256), cs, hb, hp, W, H, ms,
+                                 s->p.bloom_threshold, vec & 1);
+    for (int i = kPyrLevels; i < s->n && e == cudaSuccess; ++i)
+        e = launch_chain(k_bloom_down, grid(s->mip[i].w, s->mip[i].h), blk, cs, s->mip[i - 1], s->mip[i]);
+    for (int i = s->n - 2; i >= 0 && e == cudaSuccess; --i)
+        e = launch_chain(k_bloom_up, grid((s->mip[i].w + 1) / 2, (s->mip[i].h + 1) / 2), blk, cs, s->mip[i + 1], s->mip[i]);
+    if (e != cudaSuccess) return fail(TG_ERR_CUDA, "bloom launch failed: %s", cudaGetErrorString(e));
+    typedef void (*PostFn)(const char*, long long, char*, long long, int, int, Mip, float, float, float, int);
+    static const PostFn fns[2][3] = {{k_post<false, OUT_BGRA8>, k_post<false, OUT_RGBA8>, k_post<false, OUT_RGBA32F>},
+                                     {k_post<true, OUT_BGRA8>, k_post<true, OUT_RGBA8>, k_post<true, OUT_RGBA32F>}};
+    const int of = out->format == TG_FMT_BGRA8 ? OUT_BGRA8 : out->format == TG_FMT_RGBA8 ? OUT_RGBA8 : OUT_RGBA32F;
+    e = launch_chain(fns[h16][of], grid((W + 1) / 2, H), blk, cs, hb, hp, static_cast<char*>(out->ptr), op, W, H, s->mip[0],
+                     s->p.bloom_strength, 1.0f / float(W), 1.0f / float(H), vec);
     if (e != cudaSuccess) return fail(TG_ERR_CUDA, "post-process launch failed: %s", cudaGetErrorString(e));
     return TG_OK;
 }
