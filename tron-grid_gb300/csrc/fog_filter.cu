@@ -1,21 +1,21 @@
 // Volumetric-fog froxel filter (include/tg_fog.h) on sm_103a.
 //
-// The reference's filterMain (src/volumetric_filter.slang:142-226).  A CTA of 32 x 4
-// threads covers 32 x 8 columns of 8 consecutive slices, two vertically adjacent
-// columns per thread: the columns' camera rays and the slices' view depths are
-// computed once (they are the same for every froxel of a column / slice), then
-// for each slice the 34 x 10 halo of injected texels is staged in shared memory,
-// double-buffered (the next slice's texels are loaded while this slice is
-// computed, one barrier per slice), and each thread places its froxel centres on
-// their rays, projects them into the previous frame and fetches the history
-// trilinearly.
+// The reference's filterMain (src/volumetric_filter.slang:142-226).  A CTA covers
+// 32 x 4 columns of up to 8 consecutive slices, one thread per column: the
+// column's camera ray and the slices' view depths are computed once (they are the
+// same for every froxel of a column / slice), then for each slice the 34 x 6 halo
+// of injected texels is staged in shared memory, double-buffered (the next
+// slice's texels are loaded while this slice is computed, one barrier per slice),
+// and each thread places its froxel centre on its ray, projects it into the
+// previous frame and fetches the history trilinearly.
 //
-// What bounds it: FP32 issue.  The compulsory traffic of a 320x180x64 rgba16f
-// pass (88 MB, L2-resident) is 13 us of the 6.8 TB/s a copy reaches.  Two columns
-// per thread share four rows of the 3x3 box (6 shared loads per froxel instead of
-// 9) and give two independent chains of projections and gathers.  Measured with
-// history: 79.9 us with one column per thread, two barriers per slice and a
-// division per quotient, 61.8 us as here.
+// What bounds it: FP32 issue (about 480 instructions per froxel, the unfused
+// interpolation of eight texels the largest part).  The compulsory traffic of a
+// 320x180x64 rgba16f pass (88 MB, L2-resident) is 13 us of the 6.8 TB/s a copy
+// reaches.  Measured there, with history: 79.9 us with two barriers per slice and a
+// division per quotient, 58.3 us as here (56 registers, 9 CTAs per SM; 48
+// registers and 16 slices per CTA 64, 64 registers 58.9); two columns per thread
+// (6 shared loads per froxel instead of 9, half the CTAs) 61.8.
 //
 // Every add, multiply, divide and square root on the projection path is rounded
 // as IEEE asks (no contraction into FMA), in the order the reference writes them,
@@ -38,15 +38,15 @@
 namespace tg {
 namespace {
 
-constexpr int kFogTX = 32, kFogRows = 4, kFogR = 2;  // threads across and down, columns (in y) per thread
-constexpr int kFogTY = kFogRows * kFogR;
+constexpr int kFogTX = 32, kFogTY = 4;  // columns of a CTA (256 threads: 74 us against 60)
 constexpr int kFogSW = kFogTX + 2, kFogSH = kFogTY + 2;
-constexpr int kFogZC = 8;  // slices per CTA
+constexpr int kFogZC = 8;  // most slices per CTA (FogArgs::zc)
 
 struct FogArgs {
     float ivp[16], pvp[16], cam[3];
     float alpha, znear, zfar;
     int W, H, D, valid;
+    int zc;         // slices per CTA
     int plain_div;  // the depth range is too extreme for quotients by reciprocal
     const char* raw;
     const char* hist;
@@ -129,19 +129,20 @@ __device__ __forceinline__ float4 lerp4(float4 a, float4 b, float t)
 
 // Off: byte offsets within a volume (32 bits unless one is 4 GB or more).
 template <bool RAW16, bool OUT16, class Off>
-__global__ void __launch_bounds__(kFogTX* kFogRows) k_fog_filter(const FogArgs a)
+__global__ void __launch_bounds__(kFogTX* kFogTY, 9) k_fog_filter(const FogArgs a)
 {
     typedef Texel<RAW16> TR;
     typedef Texel<OUT16> TO;
-    constexpr int kThreads = kFogTX * kFogRows;
+    constexpr int kThreads = kFogTX * kFogTY;
     constexpr int kCells = (kFogSH * kFogSW + kThreads - 1) / kThreads;
     __shared__ float4 tile[2][kFogSH * kFogSW];
     __shared__ float view_z[kFogZC];
     pdl_begin();
-    const int x0 = blockIdx.x * kFogTX, y0 = blockIdx.y * kFogTY, z0 = blockIdx.z * kFogZC;
+    const int x0 = blockIdx.x * kFogTX, y0 = blockIdx.y * kFogTY, z0 = blockIdx.z * a.zc;
     const int tid = threadIdx.y * kFogTX + threadIdx.x;
-    const int x = x0 + threadIdx.x, yb = y0 + threadIdx.y * kFogR;
-    const int nz = min(kFogZC, a.D - z0);
+    const int x = x0 + threadIdx.x, y = y0 + threadIdx.y;
+    const bool inside = x < a.W && y < a.H;
+    const int nz = min(a.zc, a.D - z0);
     const float ratio = dv(a.zfar, a.znear);
 
     // This thread's cells of a slice's halo tile (the same in every slice), and the first slice's texels.  Cells
@@ -165,50 +166,40 @@ __global__ void __launch_bounds__(kFogTX* kFogRows) k_fog_filter(const FogArgs a
         const float tz = dv(add(float(z0 + tid), 0.5f), float(a.D));
         view_z[tid] = mul(a.znear, powf(ratio, tz));
     }
-    // Per column: the normalised camera ray through the column's NDC and its cosine to the camera axis (:83-106),
-    // and the in-grid members of its 3x3 box.
-    float ray[kFogR][3], rdf[kFogR], rrdf[kFogR], cnt[kFogR], rcnt[kFogR];
-    bool inside[kFogR];
-    float lnr = 1.f;
-    if (a.valid) lnr = logf(ratio);
-    const float rnear = __frcp_rn(a.znear), rlnr = __frcp_rn(lnr);
+    // Per column: the normalised camera ray through the column's NDC and its cosine to the camera axis (:83-106).
+    float ray[3] = {0.f, 0.f, 0.f}, rdf = 1.f, rrdf = 1.f, lnr = 1.f;
+    if (a.valid && inside) {
+        const float u = dv(add(float(x), 0.5f), float(a.W)), v = dv(add(float(y), 0.5f), float(a.H));
+        const float nx = sub(mul(u, 2.f), 1.f), ny = sub(1.f, mul(v, 2.f));
+        float nh[4], fh[4], fwd[3];
+        mat_vec(a.ivp, nx, ny, 0.f, 1.f, nh);
+        mat_vec(a.ivp, 0.f, 0.f, 0.f, 1.f, fh);
 #pragma unroll
-    for (int c = 0; c < kFogR; ++c) {
-        const int y = yb + c;
-        inside[c] = x < a.W && y < a.H;
-        rdf[c] = rrdf[c] = 1.f;
-        ray[c][0] = ray[c][1] = ray[c][2] = 0.f;
-        if (a.valid && inside[c]) {
-            const float u = dv(add(float(x), 0.5f), float(a.W)), v = dv(add(float(y), 0.5f), float(a.H));
-            const float nx = sub(mul(u, 2.f), 1.f), ny = sub(1.f, mul(v, 2.f));
-            float nh[4], fh[4], fwd[3];
-            mat_vec(a.ivp, nx, ny, 0.f, 1.f, nh);
-            mat_vec(a.ivp, 0.f, 0.f, 0.f, 1.f, fh);
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                ray[c][k] = sub(dv(nh[k], nh[3]), a.cam[k]);
-                fwd[k] = sub(dv(fh[k], fh[3]), a.cam[k]);
-            }
-            const float rl = __fsqrt_rn(add(add(mul(ray[c][0], ray[c][0]), mul(ray[c][1], ray[c][1])), mul(ray[c][2], ray[c][2])));
-            const float fl = __fsqrt_rn(add(add(mul(fwd[0], fwd[0]), mul(fwd[1], fwd[1])), mul(fwd[2], fwd[2])));
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                ray[c][k] = dv(ray[c][k], rl);
-                fwd[k] = dv(fwd[k], fl);
-            }
-            const float rd = add(add(mul(ray[c][0], fwd[0]), mul(ray[c][1], fwd[1])), mul(ray[c][2], fwd[2]));
-            rdf[c] = rd > 1e-4f ? rd : 1e-4f;
-            rrdf[c] = __frcp_rn(rdf[c]);
+        for (int k = 0; k < 3; ++k) {
+            ray[k] = sub(dv(nh[k], nh[3]), a.cam[k]);
+            fwd[k] = sub(dv(fh[k], fh[3]), a.cam[k]);
         }
-        float n = 0.f;
+        const float rl = __fsqrt_rn(add(add(mul(ray[0], ray[0]), mul(ray[1], ray[1])), mul(ray[2], ray[2])));
+        const float fl = __fsqrt_rn(add(add(mul(fwd[0], fwd[0]), mul(fwd[1], fwd[1])), mul(fwd[2], fwd[2])));
 #pragma unroll
-        for (int dy = -1; dy <= 1; ++dy)
-#pragma unroll
-            for (int dx = -1; dx <= 1; ++dx)
-                if (x + dx >= 0 && x + dx <= a.W - 1 && y + dy >= 0 && y + dy <= a.H - 1) n = add(n, 1.f);
-        cnt[c] = fmaxf(n, 1.f);
-        rcnt[c] = __frcp_rn(cnt[c]);
+        for (int k = 0; k < 3; ++k) {
+            ray[k] = dv(ray[k], rl);
+            fwd[k] = dv(fwd[k], fl);
+        }
+        rdf = add(add(mul(ray[0], fwd[0]), mul(ray[1], fwd[1])), mul(ray[2], fwd[2]));
+        rdf = rdf > 1e-4f ? rdf : 1e-4f;
+        rrdf = __frcp_rn(rdf);
+        lnr = logf(ratio);
     }
+    const float rnear = __frcp_rn(a.znear), rlnr = __frcp_rn(lnr);
+    // In-grid members of the column's 3x3 box.
+    float n = 0.f;
+#pragma unroll
+    for (int dy = -1; dy <= 1; ++dy)
+#pragma unroll
+        for (int dx = -1; dx <= 1; ++dx)
+            if (x + dx >= 0 && x + dx <= a.W - 1 && y + dy >= 0 && y + dy <= a.H - 1) n = add(n, 1.f);
+    const float cnt = fmaxf(n, 1.f), rcnt = __frcp_rn(cnt);
 
     for (int zi = 0; zi < nz; ++zi) {
         const int z = z0 + zi;
@@ -224,78 +215,69 @@ __global__ void __launch_bounds__(kFogTX* kFogRows) k_fog_filter(const FogArgs a
 #pragma unroll
             for (int e = 0; e < kCells; ++e) next[e] = cin[e] ? ld_raw<RAW16>(rs, cell[e]) : TR::zero();
         }
+        if (!inside) continue;
 
         // 1. 3x3 mean over the in-grid neighbours of the slice (:152-166), summed in the reference's order
-        float4 s[kFogR];
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int c = 0; c < kFogR; ++c) s[c] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int r = 0; r < kFogR + 2; ++r)
+        for (int dy = 0; dy < 3; ++dy)
 #pragma unroll
             for (int dx = 0; dx < 3; ++dx) {
-                const float4 q = t[(threadIdx.y * kFogR + r) * kFogSW + threadIdx.x + dx];
-#pragma unroll
-                for (int c = 0; c < kFogR; ++c)
-                    if (r >= c && r <= c + 2) s[c] = make_float4(add(s[c].x, q.x), add(s[c].y, q.y), add(s[c].z, q.z), add(s[c].w, q.w));
+                const float4 q = t[(threadIdx.y + dy) * kFogSW + threadIdx.x + dx];
+                s = make_float4(add(s.x, q.x), add(s.y, q.y), add(s.z, q.z), add(s.w, q.w));
             }
+        float4 res;
+        if (fmaxf(fmaxf(fabsf(s.x), fabsf(s.y)), fmaxf(fabsf(s.z), fabsf(s.w))) < kDivMax)
+            res = make_float4(div_count(s.x, cnt, rcnt), div_count(s.y, cnt, rcnt), div_count(s.z, cnt, rcnt),
+                              div_count(s.w, cnt, rcnt));
+        else
+            res = make_float4(dv(s.x, cnt), dv(s.y, cnt), dv(s.z, cnt), dv(s.w, cnt));
+        if (a.valid) {
+            // 2. froxel centre on the column's ray at the slice's view depth (:100-106)
+            const float tt = a.plain_div ? dv(view_z[zi], rdf) : div_by(view_z[zi], rdf, rrdf);
+            const float wx = add(a.cam[0], mul(ray[0], tt)), wy = add(a.cam[1], mul(ray[1], tt)),
+                        wz = add(a.cam[2], mul(ray[2], tt));
 
-#pragma unroll
-        for (int c = 0; c < kFogR; ++c) {
-            if (!inside[c]) continue;
-            float4 sp;
-            if (fmaxf(fmaxf(fabsf(s[c].x), fabsf(s[c].y)), fmaxf(fabsf(s[c].z), fabsf(s[c].w))) < kDivMax)
-                sp = make_float4(div_count(s[c].x, cnt[c], rcnt[c]), div_count(s[c].y, cnt[c], rcnt[c]),
-                                 div_count(s[c].z, cnt[c], rcnt[c]), div_count(s[c].w, cnt[c], rcnt[c]));
-            else
-                sp = make_float4(dv(s[c].x, cnt[c]), dv(s[c].y, cnt[c]), dv(s[c].z, cnt[c]), dv(s[c].w, cnt[c]));
-            float4 res = sp;
-            if (a.valid) {
-                // 2. froxel centre on the column's ray at the slice's view depth (:100-106)
-                const float tt = a.plain_div ? dv(view_z[zi], rdf[c]) : div_by(view_z[zi], rdf[c], rrdf[c]);
-                const float wx = add(a.cam[0], mul(ray[c][0], tt)), wy = add(a.cam[1], mul(ray[c][1], tt)),
-                            wz = add(a.cam[2], mul(ray[c][2], tt));
-
-                // 3. previous-frame froxel coordinates and rejections (:177-213)
-                float pc[4];
-                mat_vec(a.pvp, wx, wy, wz, 1.f, pc);
-                const float pz = pc[3];
-                float ndx, ndy, lt;
-                if (!a.plain_div && fmaxf(fmaxf(fabsf(pc[0]), fabsf(pc[1])), fabsf(pz)) < kDivMax) {
-                    const float rw = __frcp_rn(pz);
-                    ndx = div_by(pc[0], pz, rw);
-                    ndy = div_by(pc[1], pz, rw);
-                    lt = div_by(logf(div_by(pz, a.znear, rnear)), lnr, rlnr);
-                } else {
-                    ndx = dv(pc[0], pz);
-                    ndy = dv(pc[1], pz);
-                    lt = dv(logf(dv(pz, a.znear)), lnr);
-                }
-                const float fx = mul(add(mul(ndx, 0.5f), 0.5f), float(a.W));
-                const float fy = mul(add(mul(-ndy, 0.5f), 0.5f), float(a.H));
-                const float fz = sub(mul(lt, float(a.D)), 0.5f);
-                const bool rej = pz <= 1e-4f || pz < a.znear || pz > a.zfar || fx < 0.f || fx >= float(a.W) || fy < 0.f ||
-                                 fy >= float(a.H) || fz < 0.f || fz >= float(a.D);
-                if (!rej) {
-                    // 4. trilinear history, clamp-to-edge (:111-140), then the EMA (:216-225)
-                    const int ix = int(floorf(fx)), iy = int(floorf(fy)), iz = int(floorf(fz));
-                    const float ax = sub(fx, float(ix)), ay = sub(fy, float(iy)), az = sub(fz, float(iz));
-                    const int xa = min(max(ix, 0), a.W - 1), xb = min(max(ix + 1, 0), a.W - 1);
-                    const int ya = min(max(iy, 0), a.H - 1), yc = min(max(iy + 1, 0), a.H - 1);
-                    const int za = min(max(iz, 0), a.D - 1), zb = min(max(iz + 1, 0), a.D - 1);
-                    const Off oxa = Off(xa * TO::kBytes), oxb = Off(xb * TO::kBytes);
-                    const Off ra = Off(za) * Off(a.hist_slice) + Off(ya) * Off(a.hist_row);
-                    const Off dy = Off(yc - ya) * Off(a.hist_row), dz = Off(zb - za) * Off(a.hist_slice);
-                    typename TO::raw h[8];
-#pragma unroll
-                    for (int k = 0; k < 8; ++k)
-                        h[k] = ld_raw<OUT16>(a.hist, ra + (k & 4 ? dz : Off(0)) + (k & 2 ? dy : Off(0)) + (k & 1 ? oxb : oxa));
-                    const float4 c0 = lerp4(lerp4(TO::value(h[0]), TO::value(h[1]), ax), lerp4(TO::value(h[2]), TO::value(h[3]), ax), ay);
-                    const float4 c1 = lerp4(lerp4(TO::value(h[4]), TO::value(h[5]), ax), lerp4(TO::value(h[6]), TO::value(h[7]), ax), ay);
-                    res = lerp4(lerp4(c0, c1, az), sp, a.alpha);
-                }
+            // 3. previous-frame froxel coordinates and rejections (:177-213)
+            float pc[4];
+            mat_vec(a.pvp, wx, wy, wz, 1.f, pc);
+            const float pz = pc[3];
+            float ndx, ndy, lt;
+            if (!a.plain_div && fmaxf(fmaxf(fabsf(pc[0]), fabsf(pc[1])), fabsf(pz)) < kDivMax) {
+                const float rw = __frcp_rn(pz);
+                ndx = div_by(pc[0], pz, rw);
+                ndy = div_by(pc[1], pz, rw);
+                lt = div_by(logf(div_by(pz, a.znear, rnear)), lnr, rlnr);
+            } else {
+                ndx = dv(pc[0], pz);
+                ndy = dv(pc[1], pz);
+                lt = dv(logf(dv(pz, a.znear)), lnr);
             }
-            st_texel<OUT16>(a.out, z * a.out_slice + (yb + c) * a.out_row + x * (long long)TO::kBytes, res);
+            const float fx = mul(add(mul(ndx, 0.5f), 0.5f), float(a.W));
+            const float fy = mul(add(mul(-ndy, 0.5f), 0.5f), float(a.H));
+            const float fz = sub(mul(lt, float(a.D)), 0.5f);
+            const bool rej = pz <= 1e-4f || pz < a.znear || pz > a.zfar || fx < 0.f || fx >= float(a.W) || fy < 0.f ||
+                             fy >= float(a.H) || fz < 0.f || fz >= float(a.D);
+            if (!rej) {
+                // 4. trilinear history, clamp-to-edge (:111-140), then the EMA (:216-225)
+                const int ix = int(floorf(fx)), iy = int(floorf(fy)), iz = int(floorf(fz));
+                const float ax = sub(fx, float(ix)), ay = sub(fy, float(iy)), az = sub(fz, float(iz));
+                const int xa = min(max(ix, 0), a.W - 1), xb = min(max(ix + 1, 0), a.W - 1);
+                const int ya = min(max(iy, 0), a.H - 1), yb = min(max(iy + 1, 0), a.H - 1);
+                const int za = min(max(iz, 0), a.D - 1), zb = min(max(iz + 1, 0), a.D - 1);
+                const Off oxa = Off(xa * TO::kBytes), oxb = Off(xb * TO::kBytes);
+                const Off at = Off(za) * Off(a.hist_slice) + Off(ya) * Off(a.hist_row);
+                const Off dy = Off(yb - ya) * Off(a.hist_row), dz = Off(zb - za) * Off(a.hist_slice);
+                typename TO::raw h[8];
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+                    h[k] = ld_raw<OUT16>(a.hist, at + (k & 4 ? dz : Off(0)) + (k & 2 ? dy : Off(0)) + (k & 1 ? oxb : oxa));
+                const float4 c0 = lerp4(lerp4(TO::value(h[0]), TO::value(h[1]), ax), lerp4(TO::value(h[2]), TO::value(h[3]), ax), ay);
+                const float4 c1 = lerp4(lerp4(TO::value(h[4]), TO::value(h[5]), ax), lerp4(TO::value(h[6]), TO::value(h[7]), ax), ay);
+                res = lerp4(lerp4(c0, c1, az), res, a.alpha);
+            }
         }
+        st_texel<OUT16>(a.out, z * a.out_slice + y * a.out_row + x * (long long)TO::kBytes, res);
     }
 }
 
@@ -337,7 +319,7 @@ int tg_fog_filter(const tg_fog_filter_params* p, const tg_volume* raw, const tg_
 {
     if (!p) return fail(TG_ERR_INVALID, "null parameters");
     const uint32_t W = p->froxel_width, H = p->froxel_height, D = p->froxel_depth;
-    if (W == 0 || H == 0 || D == 0 || W > 65535u * kFogTX || H > 65535u * kFogRows || D > 65535u)
+    if (W == 0 || H == 0 || D == 0 || W > 65535u * kFogTX || H > 65535u * kFogTY || D > 65535u)
         return fail(TG_ERR_INVALID, "froxel grid %ux%ux%u outside 1..(2097120, 262140, 65535)", W, H, D);
     if (!(p->near_plane > 0.f) || !(p->far_plane > p->near_plane))
         return fail(TG_ERR_INVALID, "depth range needs 0 < near_plane < far_plane");
@@ -373,8 +355,16 @@ int tg_fog_filter(const tg_fog_filter_params* p, const tg_volume* raw, const tg_
     a.hist_slice = gh.slice;
     a.out_row = go.row;
     a.out_slice = go.slice;
-    const dim3 grid((W + kFogTX - 1) / kFogTX, (H + kFogTY - 1) / kFogTY, (D + kFogZC - 1) / kFogZC),
-        block(kFogTX, kFogRows);
+    // Slices per CTA: up to 8 share the column's set-up; a small grid takes fewer until it has 6 CTAs per SM, since its
+    // pass is then one CTA's chain of slices.
+    int dev = 0, sms = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const uint32_t tiles = ((W + kFogTX - 1) / kFogTX) * ((H + kFogTY - 1) / kFogTY);
+    a.zc = kFogZC;
+    while (a.zc > 1 && uint64_t(tiles) * ((D + a.zc - 1) / a.zc) < 6ull * sms) a.zc /= 2;
+    const dim3 grid((W + kFogTX - 1) / kFogTX, (H + kFogTY - 1) / kFogTY, (D + a.zc - 1) / a.zc),
+        block(kFogTX, kFogTY);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const bool r16 = raw->format == TG_FMT_RGBA16F, o16 = out->format == TG_FMT_RGBA16F;
     const bool wide = gr.bytes > 0xffffffffLL || gh.bytes > 0xffffffffLL;
