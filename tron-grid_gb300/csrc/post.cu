@@ -22,8 +22,8 @@
 // thread owns the 2x2 texels that share a tent, a post thread two pixels that
 // share a bloom texel (and, away from the corners, all three samples of a pixel
 // are one), and the launches overlap by programmatic dependent launch.  Measured:
-// the 3840x2160 chain (rgba16f to BGRA8) 166 -> 115 us, 1281x721 (rgba32f to
-// rgba32f) 49.8 -> 26.1 us.
+// the 3840x2160 chain (rgba16f to BGRA8) 166 -> 105 us, 1281x721 (rgba32f to
+// rgba32f) 49.8 -> 24.3 us.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -152,8 +152,11 @@ __device__ __forceinline__ C3 box4(const C3 (&c)[4])
 // Extraction and the downsample pyramid in one launch.  Mip i texel (x, y) reads exactly the 2x2 block
 // (2x, 2y) .. (2x+1, 2y+1) of mip i-1 (clamped, and the clamp never leaves the block's aligned tile because
 // mip i is floor(mip i-1 / 2) wide, or 1 wide when mip i-1 is), so a CTA that owns an aligned 32x32 tile of
-// mip 0 owns the (32 >> i)-square tile of every mip i <= 5 and builds it from shared memory, with the values
-// as the fp16 image stores them.
+// mip 0 owns the (32 >> i)-square tile of every mip i <= 5, with the values as the fp16 image stores them.
+//
+// A thread extracts the 2x2 block of mip 0 under its mip 1 texel (all 16 HDR pixels loaded up front); the next
+// two mips are exchanged between lanes (a warp's mip 1 texels are 8 x 4, lane bits x0 y0 x1 y1 x2), and only
+// the last two go through shared memory: one barrier instead of one per mip.  33.1 -> 23.8 us at 3840x2160 (under ncu).
 constexpr int kPyrT = 32;
 constexpr int kPyrLevels = 6;
 struct MipSet {
@@ -161,67 +164,89 @@ struct MipSet {
     int n;  // levels built here, 1 .. kPyrLevels
 };
 
+__device__ __forceinline__ C3 shfl_xor(C3 c, int bit)
+{
+    return {__shfl_xor_sync(0xffffffffu, c.r, bit), __shfl_xor_sync(0xffffffffu, c.g, bit), __shfl_xor_sync(0xffffffffu, c.b, bit)};
+}
+
+// The 2x2 block {(0,0), (1,0), (0,1), (1,1)} of the level below as the downsample reads it: a level one texel
+// wide or high repeats it (`w1`, `h1`).
+__device__ __forceinline__ C3 box_of(C3 c00, C3 c10, C3 c01, C3 c11, bool w1, bool h1)
+{
+    if (w1) {
+        c10 = c00;
+        c11 = c01;
+    }
+    if (h1) {
+        c01 = c00;
+        c11 = c10;
+    }
+    const C3 c[4] = {c00, c10, c01, c11};
+    return round16(box4(c));
+}
+
 template <bool HDR16>
 __global__ void __launch_bounds__(256) k_bloom_pyramid(const char* hdr, long long pitch, int W, int H, MipSet ms, float thr, int vec)
 {
-    __shared__ float sa[3][kPyrT * kPyrT];  // ping-pong tiles of one mip level, one plane per channel
-    __shared__ float sb[3][kPyrT * kPyrT];
-    const int tid = threadIdx.x;
-    const int X0 = blockIdx.x * kPyrT, Y0 = blockIdx.y * kPyrT;
+    __shared__ C3 s3[16];  // the CTA's 4x4 texels of mip 3
     pdl_begin();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // mip 1 texel of this thread: warps 2 across, 4 down
+    const int tx = (warp & 1) * 8 + (lane & 1) + ((lane >> 1) & 2) + ((lane >> 2) & 4);
+    const int ty = (warp >> 1) * 4 + ((lane >> 1) & 1) + ((lane >> 2) & 2);
+    const int x1 = blockIdx.x * (kPyrT / 2) + tx, y1 = blockIdx.y * (kPyrT / 2) + ty;
+    const Mip m0 = ms.m[0];
     // every HDR load of the thread's four texels is issued before the first is used
-    constexpr int kPer = kPyrT * kPyrT / 256;
-    C3 in[kPer][4];
+    C3 in[4][4];
 #pragma unroll
-    for (int e = 0; e < kPer; ++e) {
-        const int k = tid + e * 256;
-        const int x = min(X0 + k % kPyrT, ms.m[0].w - 1), y = min(Y0 + k / kPyrT, ms.m[0].h - 1);
-        C3 row[2];
+    for (int q = 0; q < 4; ++q) {
+        const int x = min(2 * x1 + (q & 1), m0.w - 1), y = min(2 * y1 + (q >> 1), m0.h - 1);
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
+            C3 row[2];
             ld_hdr2<HDR16>(hdr, pitch, min(2 * x, W - 1), min(2 * x + 1, W - 1), min(2 * y + j, H - 1), vec, row);
-            in[e][2 * j] = row[0];
-            in[e][2 * j + 1] = row[1];
+            in[q][2 * j] = row[0];
+            in[q][2 * j + 1] = row[1];
         }
     }
+    C3 t0[4];
 #pragma unroll
-    for (int e = 0; e < kPer; ++e) {
-        const int k = tid + e * 256;
-        const int x = X0 + k % kPyrT, y = Y0 + k / kPyrT;
-        if (x >= ms.m[0].w || y >= ms.m[0].h) continue;
-        const C3 c = round16(extract_texel(in[e], thr));
-        st_h4(ms.m[0].p, (long long)y * ms.m[0].w + x, c);
-        sa[0][k] = c.r;
-        sa[1][k] = c.g;
-        sa[2][k] = c.b;
+    for (int q = 0; q < 4; ++q) {
+        t0[q] = round16(extract_texel(in[q], thr));
+        const int x = 2 * x1 + (q & 1), y = 2 * y1 + (q >> 1);
+        if (x < m0.w && y < m0.h) st_h4(m0.p, (long long)y * m0.w + x, t0[q]);
     }
-    float(*cur)[kPyrT * kPyrT] = sa;
-    float(*nxt)[kPyrT * kPyrT] = sb;
-    int side = kPyrT;
-    for (int i = 1; i < ms.n; ++i) {
-        __syncthreads();
-        const Mip s = ms.m[i - 1], d = ms.m[i];
-        const int ns = side >> 1, sx0 = X0 >> (i - 1), sy0 = Y0 >> (i - 1), dx0 = X0 >> i, dy0 = Y0 >> i;
-        for (int k = tid; k < ns * ns; k += 256) {
-            const int x = dx0 + k % ns, y = dy0 + k / ns;
-            if (x >= d.w || y >= d.h) continue;
-            C3 c[4];
+    if (ms.n < 2) return;
+    // (texels outside a mip hold values that no texel inside the next one reads)
+    const C3 c1 = box_of(t0[0], t0[1], t0[2], t0[3], m0.w == 1, m0.h == 1);
+    if (x1 < ms.m[1].w && y1 < ms.m[1].h) st_h4(ms.m[1].p, (long long)y1 * ms.m[1].w + x1, c1);
+    if (ms.n < 3) return;
+    // mips 2 and 3: the lane whose two bits of the pair are 0 holds the block's first texel
+    C3 c = c1;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int j = (min(2 * y + (q >> 1), s.h - 1) - sy0) * side + (min(2 * x + (q & 1), s.w - 1) - sx0);
-                c[q] = {cur[0][j], cur[1][j], cur[2][j]};
-            }
-            const C3 v = round16(box4(c));
-            st_h4(d.p, (long long)y * d.w + x, v);
-            nxt[0][k] = v.r;
-            nxt[1][k] = v.g;
-            nxt[2][k] = v.b;
-        }
-        float(*t)[kPyrT * kPyrT] = cur;
-        cur = nxt;
-        nxt = t;
-        side = ns;
+    for (int i = 2; i < 4; ++i) {
+        if (ms.n <= i) return;
+        const int bx = i == 2 ? 1 : 4, by = i == 2 ? 2 : 8;
+        const C3 r = shfl_xor(c, bx), d = shfl_xor(c, by), rd = shfl_xor(r, by);
+        c = box_of(c, r, d, rd, ms.m[i - 1].w == 1, ms.m[i - 1].h == 1);
+        const int x = x1 >> (i - 1), y = y1 >> (i - 1);
+        const bool first = (lane & (i == 2 ? 3 : 15)) == 0;
+        if (first && x < ms.m[i].w && y < ms.m[i].h) st_h4(ms.m[i].p, (long long)y * ms.m[i].w + x, c);
     }
+    if (ms.n < 5) return;
+    if ((lane & 15) == 0) s3[(ty >> 2) * 4 + (tx >> 2)] = c;
+    __syncthreads();
+    if (warp != 0) return;
+    // mips 4 (lanes 0 .. 3) and 5 (lane 0)
+    const int i4 = (lane & 1) * 2 + ((lane >> 1) & 1) * 8;
+    const C3 c4 = box_of(s3[i4], s3[i4 + 1], s3[i4 + 4], s3[i4 + 5], ms.m[3].w == 1, ms.m[3].h == 1);
+    const int x4 = blockIdx.x * 2 + (lane & 1), y4 = blockIdx.y * 2 + ((lane >> 1) & 1);
+    if (lane < 4 && x4 < ms.m[4].w && y4 < ms.m[4].h) st_h4(ms.m[4].p, (long long)y4 * ms.m[4].w + x4, c4);
+    if (ms.n < 6) return;
+    const C3 r = shfl_xor(c4, 1), d = shfl_xor(c4, 2), rd = shfl_xor(r, 2);
+    const C3 c5 = box_of(c4, r, d, rd, ms.m[4].w == 1, ms.m[4].h == 1);
+    if (lane == 0 && int(blockIdx.x) < ms.m[5].w && int(blockIdx.y) < ms.m[5].h)
+        st_h4(ms.m[5].p, (long long)blockIdx.y * ms.m[5].w + blockIdx.x, c5);
 }
 
 __global__ void __launch_bounds__(kPostTX* kPostTY) k_bloom_down(Mip s, Mip d)
