@@ -192,23 +192,25 @@ int validate_params(const tg_svgf_params& p)
 } // namespace tg
 
 namespace tg {
-// Output rows per thread of the tiled a-trous kernels: FULL (kLevelR) and
-// REF_EXACT (kRefR).
+// Output rows per thread of the plain-load a-trous kernels.
 constexpr int kLevelR = 2;
-#ifndef TG_REF_R
-#define TG_REF_R 2
-#endif
-constexpr int kRefR = TG_REF_R;
 
 typedef void (*LevelTmaFn)(FullArgs, LevelArgs, LevelGeom, const CUtensorMap, const CUtensorMap);
 typedef void (*LevelTiledFn)(FullArgs, LevelGeom);
 
-// The FULL a-trous kernel for a level: FP16 or FP32 storage, VAR = false at the
+// The FULL a-trous kernel for a level of R rows per thread: VAR = false at the
 // last level (it writes only colour), PL at level 0 (staged from the planes).
-template <bool PL> LevelTmaFn level_tma_kernel(bool f16, bool last)
+template <int ST, int R> LevelTmaFn level_tma_kernel_r(bool pl, bool last)
 {
-    if (f16) return last ? k_full_level_tma<ST_FP16, kLevelR, false, PL> : k_full_level_tma<ST_FP16, kLevelR, true, PL>;
-    return last ? k_full_level_tma<ST_FP32, kLevelR, false, PL> : k_full_level_tma<ST_FP32, kLevelR, true, PL>;
+    if (pl) return last ? k_full_level_tma<ST, R, false, true> : k_full_level_tma<ST, R, true, true>;
+    return last ? k_full_level_tma<ST, R, false, false> : k_full_level_tma<ST, R, true, false>;
+}
+LevelTmaFn level_tma_kernel(bool f16, bool pl, bool last, int rows)
+{
+    if (rows == 3) return f16 ? level_tma_kernel_r<ST_FP16, 3>(pl, last) : level_tma_kernel_r<ST_FP32, 3>(pl, last);
+    // (two rows: never the last level, level_rows)
+    if (f16) return pl ? k_full_level_tma<ST_FP16, 2, true, true> : k_full_level_tma<ST_FP16, 2, true, false>;
+    return pl ? k_full_level_tma<ST_FP32, 2, true, true> : k_full_level_tma<ST_FP32, 2, true, false>;
 }
 template <bool PL> LevelTiledFn level_tiled_kernel(bool f16, bool last)
 {
@@ -240,6 +242,8 @@ struct tg_svgf {
     int* d_err = nullptr;  // device error word of bounded waits
     int flags = 0;
     bool tma = false;                // a-trous tiles staged by TMA
+    int rows[10];                    // output rows per thread of each FULL level's TMA kernel (level_rows)
+    int ref_r = 2;                   // output rows per thread of the REF_EXACT chain (ref_rows)
     CUtensorMap tmaps[10];           // per level: the level's input records
     bool tma0 = false;               // level 0 staged by TMA from the tc and guide planes
     CUtensorMap tm_tc, tm_guide[2];  // row-major tc and guide[parity] (level 0 reads these, not records)
@@ -371,8 +375,7 @@ void build_ref_maps(tg_svgf* s, EncodeTiledFn enc)
         const cuuint64_t planes = cuuint64_t(1) << (2 * lv);
         const cuuint64_t dim[3] = {f16 ? cuuint64_t(L.pw) : 4ull * L.pw, cuuint64_t(L.ph), planes};
         const cuuint64_t str[2] = {tb * L.pw, tb * L.pw * L.ph};
-        const cuuint32_t box[3] = {f16 ? cuuint32_t(LevelTile<kRefR>::SW) : 4u * LevelTile<kRefR>::SW,
-                                   LevelTile<kRefR>::SH, 1};
+        const cuuint32_t box[3] = {f16 ? cuuint32_t(kLvTX + 4) : 4u * (kLvTX + 4), cuuint32_t(kLvRows * s->ref_r + 4), 1};
         const cuuint32_t es[3] = {1, 1, 1};
         const CUresult r = enc(&s->ref_lv[lv], f16 ? CU_TENSOR_MAP_DATA_TYPE_UINT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
                                base, dim, str, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -396,8 +399,7 @@ bool ref_input_map(tg_svgf* s, const tg_image& im)
     const bool h = tb == 8;
     const cuuint64_t dim[2] = {h ? cuuint64_t(s->w) : 4ull * s->w, s->h};
     const cuuint64_t str[1] = {cuuint64_t(pitch)};
-    const cuuint32_t box[2] = {h ? cuuint32_t(LevelTile<kRefR>::SW) : 4u * LevelTile<kRefR>::SW,
-                               LevelTile<kRefR>::SH};
+    const cuuint32_t box[2] = {h ? cuuint32_t(kLvTX + 4) : 4u * (kLvTX + 4), cuuint32_t(kLvRows * s->ref_r + 4)};
     const cuuint32_t es[2] = {1, 1};
     if (enc(&s->ref_in, h ? CU_TENSOR_MAP_DATA_TYPE_UINT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, im.ptr, dim, str, box,
             es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -413,6 +415,8 @@ bool ref_input_map(tg_svgf* s, const tg_image& im)
 void build_tensor_maps(tg_svgf* s)
 {
     s->tma = false;
+    s->ref_r = ref_rows(int(s->w), int(s->h));
+    for (int lv = 0; lv < 10; ++lv) s->rows[lv] = level_rows(int(s->w), int(s->h), lv == s->p.levels - 1);
     for (bool& ok : s->ref_lv_ok) ok = false;
     s->ref_in_ok = false;
     if (s->flags & TG_SVGF_FLAG_NO_TMA) return;
@@ -423,19 +427,22 @@ void build_tensor_maps(tg_svgf* s)
         s->tma = true;  // interior tiles of the later passes (where their planes allow) and of the first pass
         return;
     }
-    CUtensorMap maps[kFullMaps];
-    const unsigned m = full_level_maps(s->p, s->w, s->h, kLevelR, s->colA, s->colB, s->tc, s->guide[0], s->guide[1], maps);
-    for (int lv = 1; lv < s->p.levels; ++lv) {
-        if (!((m >> lv) & 1u)) return;
-        s->tmaps[lv] = maps[2 + lv];
+    for (int R = 2; R <= 3; ++R) {
+        CUtensorMap maps[kFullMaps];
+        const unsigned m = full_level_maps(s->p, s->w, s->h, R, s->colA, s->colB, s->tc, s->guide[0], s->guide[1], maps);
+        for (int lv = 1; lv < s->p.levels; ++lv) {
+            if (!((m >> lv) & 1u)) return;
+            if (s->rows[lv] == R) s->tmaps[lv] = maps[2 + lv];
+        }
+        if (s->rows[0] != R) continue;
+        s->tma0 = m & 1u;
+        if (s->tma0) {
+            s->tm_tc = maps[0];
+            s->tm_guide[0] = maps[1];
+            s->tm_guide[1] = maps[2];
+        }
     }
     s->tma = true;
-    s->tma0 = m & 1u;
-    if (s->tma0) {
-        s->tm_tc = maps[0];
-        s->tm_guide[0] = maps[1];
-        s->tm_guide[1] = maps[2];
-    }
 }
 
 void free_buffers(tg_svgf* s)
@@ -624,14 +631,18 @@ int launch_frame(tg_svgf* s, const tg_svgf_inputs* in, const tg_svgf_outputs* ou
         if (ref_input_map(s, in->radiance)) maps.first = &s->ref_in;
         for (int L = 1; L < levels && L < 10; ++L)
             if (s->ref_lv_ok[L]) maps.level[L] = &s->ref_lv[L];
-        enqueue_ref_chain<kRefR>(a, s->colA, s->colB, levels, f16, stream, maps, [&](bool first, auto body) {
+        auto hook = [&](bool first, auto body) {
             const bool last = lv == levels - 1;
             // compulsory bytes: the fused pass reads radiance and moments_prev and writes moments_curr; every
             // pass reads its input image and writes its output (the caller's image at the last pass)
             const double bytes = npx * ((first ? rb + 2 * mm : c4) + (last ? ob : c4));
             launch(s, stream, first ? F_REF_FIRST : F_REF_LEVEL, bytes, body);
             ++lv;
-        });
+        };
+        if (s->ref_r == 3)
+            enqueue_ref_chain<3>(a, s->colA, s->colB, levels, f16, stream, maps, hook);
+        else
+            enqueue_ref_chain<2>(a, s->colA, s->colB, levels, f16, stream, maps, hook);
     } else {
         FullArgs a{};
         a.w = int(s->w);
@@ -693,23 +704,18 @@ int launch_frame(tg_svgf* s, const tg_svgf_inputs* in, const tg_svgf_outputs* ou
             // variance plane (or the output) out; level 0 reads tc (colour and length), guide and variance
             // plane instead of records and also writes the history
             const double lb = (lv == 0 ? c4 + gb : rb) + vb + 8 + (a.last ? ob : rb + vb) + (lv == 0 ? c4 : 0);
-            const LevelGeom lg = level_geom(a.w, a.h, a.stride, kLevelR);
-            const dim3 lgrid(level_blocks(lg)), lblk(kLvTX, kLvRows);
+            const bool pl = lv == 0, tma = s->tma && (!pl || s->tma0);
+            const int rows = tma ? s->rows[lv] : kLevelR;
+            const LevelGeom lg = level_geom(a.w, a.h, a.stride, rows);
+            const dim3 lgrid = level_grid(lg), lblk(kLvTX, kLvRows);
             // the last level writes only colour: its kernels leave out the variance propagation
             launch(s, stream, F_FULL_LEVEL, npx * lb, [&] {
-                const bool pl = lv == 0;
-                if (s->tma && (!pl || s->tma0)) {
-                    const LevelArgs la = level_args_of(a);
-                    if (pl)
-                        launch_chain(level_tma_kernel<true>(f16, a.last), lgrid, lblk, stream, a, la, lg, s->tm_tc,
-                                     s->tm_guide[cur]);
-                    else
-                        launch_chain(level_tma_kernel<false>(f16, a.last), lgrid, lblk, stream, a, la, lg, s->tmaps[lv],
-                                     s->tmaps[lv]);
-                } else {
+                if (tma)
+                    launch_chain(level_tma_kernel(f16, pl, a.last, rows), lgrid, lblk, stream, a, level_args_of(a), lg,
+                                 pl ? s->tm_tc : s->tmaps[lv], pl ? s->tm_guide[cur] : s->tmaps[lv]);
+                else
                     launch_chain(pl ? level_tiled_kernel<true>(f16, a.last) : level_tiled_kernel<false>(f16, a.last), lgrid,
                                  lblk, stream, a, lg);
-                }
             });
             void* t = src;
             src = oth;

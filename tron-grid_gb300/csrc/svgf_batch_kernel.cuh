@@ -181,11 +181,11 @@ __global__ void __launch_bounds__(kLvTX* kLvRows, 6) k_batch_step(const char* __
                 const LevelGeom g = level_geom(a.w, a.h, 1 << L, R);
                 // level 0 stages from the planes; the last level writes only colour
                 if (L == 0)
-                    full_level_tile<ST, R, true, true>(a, lv, g, local, sm);
+                    full_level_tile<ST, R, true, true>(a, lv, g, tile_of_id<R>(g, local), sm);
                 else if (lv.last)
-                    full_level_tile<ST, R, false, false>(a, lv, g, local, sm);
+                    full_level_tile<ST, R, false, false>(a, lv, g, tile_of_id<R>(g, local), sm);
                 else
-                    full_level_tile<ST, R, true, false>(a, lv, g, local, sm);
+                    full_level_tile<ST, R, true, false>(a, lv, g, tile_of_id<R>(g, local), sm);
                 __syncthreads();
             }
         }
@@ -260,7 +260,8 @@ __global__ void __launch_bounds__(kLvTX* kLvRows, LevelOcc<R>::kCtas) k_ms_level
     lv.last = L == hd->levels - 1;
     lv.lin = res_layout(a.w, a.h, L);
     lv.lout = res_layout(a.w, a.h, L + 1);
-    full_level_tile<ST, R, VAR, PL>(a, lv, level_geom(a.w, a.h, 1 << L, R), item - pf[j], sm);
+    const LevelGeom g = level_geom(a.w, a.h, 1 << L, R);
+    full_level_tile<ST, R, VAR, PL>(a, lv, g, tile_of_id<R>(g, item - pf[j]), sm);
 }
 
 // The same stage with each stream's tiles staged by TMA through `maps` where
@@ -294,9 +295,9 @@ __global__ void __launch_bounds__(kLvTX* kLvRows, LevelOcc<R>::kCtas)
         // level 0 stages from the tc plane and this step's guide plane, the others from their records
         const CUtensorMap* tm = PL ? &maps.m[3 * e.tma_slot] : &maps.m[e.tma_slot];
         const CUtensorMap* tm2 = PL ? &maps.m[3 * e.tma_slot + 1 + e.guide_k] : tm;
-        full_level_tile_tma<ST, R, VAR, PL>(a, lv, g, item - pf[j], sm, bar, tm, tm2);
+        full_level_tile_tma<ST, R, VAR, PL>(a, lv, g, tile_of_id<R>(g, item - pf[j]), sm, bar, tm, tm2);
     } else {
-        full_level_tile<ST, R, VAR, PL>(a, lv, g, item - pf[j], sm);
+        full_level_tile<ST, R, VAR, PL>(a, lv, g, tile_of_id<R>(g, item - pf[j]), sm);
     }
 }
 

@@ -25,8 +25,10 @@ struct ResLayout {
 
 __device__ __forceinline__ size_t res_idx(const ResLayout& L, int x, int y)
 {
-    const int m = (1 << L.lg) - 1;
-    return (size_t(((y & m) << L.lg) + (x & m)) * L.ph + (y >> L.lg)) * L.pw + (x >> L.lg);
+    // (fewer than 2^31 cells: images are at most 32768 x 32768)
+    const unsigned m = (1u << L.lg) - 1u;
+    return ((((unsigned(y) & m) << L.lg) + (unsigned(x) & m)) * unsigned(L.ph) + (unsigned(y) >> L.lg)) * unsigned(L.pw) +
+           (unsigned(x) >> L.lg);
 }
 
 __host__ __device__ inline ResLayout res_layout(int w, int h, int lg)

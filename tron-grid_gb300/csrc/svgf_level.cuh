@@ -63,10 +63,25 @@ template <int R> struct LevelTile {
 // CTAs per SM the level kernels are compiled for: at R = 2 eight CTAs of 128
 // threads (32 warps, 64 registers a thread) hide the tap loop's latencies and
 // the tile waits better than four of 256 threads (2% slower per level), two of
-// 512 (15% slower) or 256-thread CTAs at 80 registers.
+// 512 (15% slower) or 256-thread CTAs at 80 registers; at R = 3 five (96
+// registers; the last level too: six at 80 registers were 4% slower).
 template <int R> struct LevelOcc {
-    static constexpr int kCtas = R <= 2 ? 8 : 4;
+    static constexpr int kCtas = R <= 2 ? 8 : 5;
 };
+
+// Output rows per thread of a single-stream FULL level.  Three rows need 12%
+// fewer instructions and a fifth less shared-memory traffic per output, but only
+// five CTAs are resident, so a level of few waves loses more to its last one:
+// 3840x2160 187 / 174 / 180 / 190 us for levels 0 to 3 against 193 / 180 / 183 /
+// 188 with two rows (28 waves), 1920x1080 52 / 49 / 53.5 / 59 against 52 / 49 /
+// 50 / 56 (7 waves).  The last level writes only colour and is bound by its
+// scattered stores more than by its registers: three rows are faster from
+// 640x360 (12.8 against 13.2 us) to 3840x2160 (207 against 222).
+__host__ inline int level_rows(int w, int h, bool last)
+{
+    const long long tiles = (long long)((w + kLvTX - 1) / kLvTX) * ((h + 3 * kLvRows - 1) / (3 * kLvRows));
+    return last || tiles >= 16 * 5 * 152 ? 3 : 2;
+}
 
 // Staged tile of one level: X0 = (r, g, b, variance), X1 = (unit normal, depth),
 // XL = luminance.  A TMA box must land on a 128-byte boundary: X0 and X1 start
@@ -95,6 +110,36 @@ __device__ __forceinline__ void level_block(const LevelGeom& g, int bid, int TX,
     i0 = int(tile - ty * unsigned(g.tiles_x)) * TX;
     j0 = int(ty) * TY;
 }
+
+// The same tile from a 2-D grid (level_grid), without the division.
+__device__ __forceinline__ void level_block2(const LevelGeom& g, int TX, int TY, int& ra, int& rb, int& i0, int& j0)
+{
+    const unsigned res = blockIdx.x & ((1u << (2 * g.lg)) - 1u);
+    ra = int(res & unsigned(g.s - 1));
+    rb = int(res >> g.lg);
+    i0 = int(blockIdx.x >> (2 * g.lg)) * TX;
+    j0 = int(blockIdx.y) * TY;
+}
+
+struct TileAt {
+    int ra, rb, i0, j0;
+};
+
+template <int R> __device__ __forceinline__ TileAt tile_of_grid(const LevelGeom& g)
+{
+    TileAt t;
+    level_block2(g, LevelTile<R>::TX, LevelTile<R>::TY, t.ra, t.rb, t.i0, t.j0);
+    return t;
+}
+
+template <int R> __device__ __forceinline__ TileAt tile_of_id(const LevelGeom& g, int bid)
+{
+    TileAt t;
+    level_block(g, bid, LevelTile<R>::TX, LevelTile<R>::TY, t.ra, t.rb, t.i0, t.j0);
+    return t;
+}
+
+__host__ inline dim3 level_grid(const LevelGeom& g) { return dim3(unsigned(g.s * g.s) * g.tiles_x, g.tiles_y); }
 
 // ------------------------------------------------------------------ FULL ----
 
@@ -375,12 +420,12 @@ __device__ __forceinline__ void level_tile_body(const FullArgs& a, const LevelAr
     level_compute<ST, R, VAR, IN>(a, lv, g, ra, rb, i0, j0, pre, sm);
 }
 
+// The tile at (t.i0, t.j0) of residue (t.ra, t.rb).
 template <int ST, int R, bool VAR = true, bool PL = false>
-__device__ __forceinline__ void full_level_tile(const FullArgs& a, const LevelArgs& lv, const LevelGeom& g, int bid,
+__device__ __forceinline__ void full_level_tile(const FullArgs& a, const LevelArgs& lv, const LevelGeom& g, const TileAt& t,
                                                 LevelSmem<R>& sm)
 {
-    int ra, rb, i0, j0;
-    level_block(g, bid, LevelTile<R>::TX, LevelTile<R>::TY, ra, rb, i0, j0);
+    const int ra = t.ra, rb = t.rb, i0 = t.i0, j0 = t.j0;
     if (tile_interior<R>(a, g.s, ra, rb, i0, j0))
         level_tile_body<ST, R, VAR, PL, true>(a, lv, g, ra, rb, i0, j0, sm);
     else
@@ -392,7 +437,7 @@ __global__ void __launch_bounds__(kLvTX* kLvRows, LevelOcc<R>::kCtas) k_full_lev
 {
     __shared__ LevelSmem<R> sm;
     pdl_begin();
-    full_level_tile<ST, R, VAR, PL>(a, level_args_of(a), g, blockIdx.x, sm);
+    full_level_tile<ST, R, VAR, PL>(a, level_args_of(a), g, tile_of_grid<R>(g), sm);
 }
 
 // ------------------------------------------------------- TMA-staged level ----
@@ -411,18 +456,23 @@ constexpr long long kTmaWaitCycles = 2000000000LL;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
 
+__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t phase)
+{
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok)
+                 : "r"(bar), "r"(phase)
+                 : "memory");
+    return ok != 0;
+}
+
 __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t phase)
 {
+    if (mbar_try_wait(bar, phase)) return true;  // (suspends for a while by itself)
     const long long t0 = clock64();
-    for (;;) {
-        uint32_t ok;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(ok)
-                     : "r"(bar), "r"(phase)
-                     : "memory");
-        if (ok) return true;
+    while (!mbar_try_wait(bar, phase))
         if (clock64() - t0 > kTmaWaitCycles) return false;
-    }
+    return true;
 }
 
 // Issues the halo box of the tile at (ra, rb, i0, j0) into `sm` (one thread).
@@ -561,16 +611,15 @@ __device__ __forceinline__ void tma_tile_body(const FullArgs& a, const LevelArgs
 // records, tc through `tm` and guide_cur through `tm2`, and each staged cell's
 // variance comes from the variance plane, loaded before the wait.  Other levels
 // read `tm` only.
-// One tile `bid` of a level staged by TMA through maps `tm` / `tm2` (kernel
+// One tile of a level staged by TMA through maps `tm` / `tm2` (kernel
 // parameters).
 template <int ST, int R, bool VAR, bool PL>
-__device__ __forceinline__ void full_level_tile_tma(const FullArgs& a, const LevelArgs& lv, const LevelGeom& g, int bid,
-                                                    LevelSmem<R>& sm, uint64_t& bar, const CUtensorMap* tm,
+__device__ __forceinline__ void full_level_tile_tma(const FullArgs& a, const LevelArgs& lv, const LevelGeom& g,
+                                                    const TileAt& t, LevelSmem<R>& sm, uint64_t& bar, const CUtensorMap* tm,
                                                     const CUtensorMap* tm2)
 {
     typedef LevelTile<R> T;
-    int ra, rb, i0, j0;
-    level_block(g, bid, T::TX, T::TY, ra, rb, i0, j0);
+    const int ra = t.ra, rb = t.rb, i0 = t.i0, j0 = t.j0;
     const int tid = threadIdx.y * kLvTX + threadIdx.x;
     const uint32_t ubar = smem_u32(&bar);
     if (tid == 0) {
@@ -594,7 +643,7 @@ __global__ void __launch_bounds__(kLvTX* kLvRows, LevelOcc<R>::kCtas)
     __shared__ LevelSmem<R> sm;
     __shared__ __align__(8) uint64_t bar;
     pdl_begin();
-    full_level_tile_tma<ST, R, VAR, PL>(a, lv, g, blockIdx.x, sm, bar, &tm, &tm2);
+    full_level_tile_tma<ST, R, VAR, PL>(a, lv, g, tile_of_grid<R>(g), sm, bar, &tm, &tm2);
 }
 
 // ------------------------------------------------------------- REF-EXACT ----
@@ -806,22 +855,28 @@ __device__ __forceinline__ void ref_first_tile(const RefArgs& a, int i0, int j0,
     ref_taps_out<ST, R>(a, 1, 0, 0, i0, j0, ca, valid, sA);
 }
 
-// CTAs per SM the REF_EXACT kernels are compiled for: 12 of 128 threads (40
-// registers a thread, 48 warps).  48 warps measured 14% faster per 4K frame
-// than the 40 that 42 registers allowed; 12 CTAs of 128 threads ran as fast as
-// 6 of 256; 3 rows per thread was slower.
-#ifndef TG_REF_CTAS
-#define TG_REF_CTAS 12
-#endif
-#ifndef TG_REF_FIRST_CTAS
-#define TG_REF_FIRST_CTAS TG_REF_CTAS
-#endif
+// CTAs per SM the REF_EXACT kernels are compiled for: at R = 2, 12 of 128
+// threads (40 registers a thread, 48 warps), which ran as fast as 6 of 256; at
+// R = 3, 10 (48 registers; 12 at 40 registers were 6% slower).
+template <int R> struct RefOcc {
+    static constexpr int kCtas = R <= 2 ? 12 : 10;
+};
+
+// Output rows per thread of a REF_EXACT chain: three share each staged texel and
+// the per-thread work among more outputs (3840x2160, binary16 images: 223 us
+// against 238 with two rows), two leave a small frame more CTAs (640x360: 19
+// against 22 us; even at 1280x720).
+__host__ inline int ref_rows(int w, int h)
+{
+    const long long tiles = (long long)((w + kLvTX - 1) / kLvTX) * ((h + 3 * kLvRows - 1) / (3 * kLvRows));
+    return tiles >= 10 * 152 ? 3 : 2;
+}
 
 // use_tma: interior tiles are staged through `tm`, a 2-D map over the caller's
 // radiance ({8-byte texel, row} for RGBA16F, {float, row} for RGBA32F);
 // border tiles (clamped taps) and use_tma == 0 stage with plain loads.
 template <int ST, int R>
-__global__ void __launch_bounds__(kLvTX* kLvRows, TG_REF_FIRST_CTAS)
+__global__ void __launch_bounds__(kLvTX* kLvRows, RefOcc<R>::kCtas)
     k_ref_first(RefArgs a, LevelGeom g, const __grid_constant__ CUtensorMap tm, int use_tma)
 {
     typedef LevelTile<R> T;
@@ -829,8 +884,8 @@ __global__ void __launch_bounds__(kLvTX* kLvRows, TG_REF_FIRST_CTAS)
     __shared__ __align__(128) float4 land[T::N];
     __shared__ __align__(8) uint64_t bar;
     pdl_begin();
-    const int i0 = int(blockIdx.x % unsigned(g.tiles_x)) * T::TX;
-    const int j0 = int(blockIdx.x / unsigned(g.tiles_x)) * T::TY;
+    const int i0 = int(blockIdx.x) * T::TX;
+    const int j0 = int(blockIdx.y) * T::TY;
     const bool in = ref_tile_interior<R>(a.w, a.h, 1, 0, 0, i0, j0);
     if (in && use_tma) {
         const uint32_t ubar = smem_u32(&bar);
@@ -906,7 +961,7 @@ __device__ __forceinline__ void ref_level_tile(const RefArgs& a, int s, int ra, 
 // residue planes ({8-byte texel, row, plane} for fp16 images, {float, row,
 // plane} for fp32 ones); border tiles and use_tma == 0 stage with plain loads.
 template <int ST, int R>
-__global__ void __launch_bounds__(kLvTX* kLvRows, TG_REF_CTAS)
+__global__ void __launch_bounds__(kLvTX* kLvRows, RefOcc<R>::kCtas)
     k_ref_level(RefArgs a, LevelGeom g, const __grid_constant__ CUtensorMap tm, int use_tma)
 {
     typedef LevelTile<R> T;
@@ -915,7 +970,7 @@ __global__ void __launch_bounds__(kLvTX* kLvRows, TG_REF_CTAS)
     __shared__ __align__(8) uint64_t bar;
     pdl_begin();
     int ra, rb, i0, j0;
-    level_block(g, blockIdx.x, T::TX, T::TY, ra, rb, i0, j0);
+    level_block2(g, T::TX, T::TY, ra, rb, i0, j0);
     const bool in = ref_tile_interior<R>(a.w, a.h, g.s, ra, rb, i0, j0);
     if (in && use_tma) {
         const uint32_t ubar = smem_u32(&bar);
@@ -981,7 +1036,7 @@ void enqueue_ref_chain(RefArgs a, void* wa, void* wb, int levels, bool f16, cuda
     hook(true, [&] {
         const CUtensorMap& m = maps.first ? *maps.first : none;
         const int t = maps.first != nullptr;
-        launch_chain(f16 ? k_ref_first<ST_FP16, R> : k_ref_first<ST_FP32, R>, dim3(level_blocks(g0)), blk, stream, a, g0,
+        launch_chain(f16 ? k_ref_first<ST_FP16, R> : k_ref_first<ST_FP32, R>, level_grid(g0), blk, stream, a, g0,
                      m, t);
     });
     void* src = wb;
@@ -997,7 +1052,7 @@ void enqueue_ref_chain(RefArgs a, void* wa, void* wb, int levels, bool f16, cuda
         hook(false, [&] {
             const CUtensorMap& m = maps.level[lv] ? *maps.level[lv] : none;
             const int t = maps.level[lv] != nullptr;
-            launch_chain(f16 ? k_ref_level<ST_FP16, R> : k_ref_level<ST_FP32, R>, dim3(level_blocks(g)), blk, stream, a,
+            launch_chain(f16 ? k_ref_level<ST_FP16, R> : k_ref_level<ST_FP32, R>, level_grid(g), blk, stream, a,
                          g, m, t);
         });
         void* t = src;

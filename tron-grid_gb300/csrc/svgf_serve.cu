@@ -463,7 +463,7 @@ void launch_plain(tg_svgf_server* sv, Sess& s)
         a.lin = res_layout(a.w, a.h, lv);
         a.lout = res_layout(a.w, a.h, lv + 1);
         const LevelGeom g = level_geom(a.w, a.h, a.stride, kR);
-        const dim3 lgrid(level_blocks(g)), lblk(kLvTX, kLvRows);
+        const dim3 lgrid = level_grid(g), lblk(kLvTX, kLvRows);
         // level 0 stages from the planes, the last level writes only colour; tiles are staged by TMA where the
         // session's maps were encoded, as the single-stream path does
         if ((s.tma_mask >> lv) & 1u) {
