@@ -239,7 +239,7 @@ struct tg_svgf {
     void* colB = nullptr;
     float2* grad = nullptr;
     int* fb_flags = nullptr;
-    int* d_err = nullptr;  // device error word of bounded waits
+    int* d_err = nullptr;  // device error word of bounded waits, then (FULL) the counter of fallback blocks
     int flags = 0;
     bool tma = false;                // a-trous tiles staged by TMA
     int rows[10];                    // output rows per thread of each FULL level's TMA kernel (level_rows)
@@ -318,7 +318,7 @@ void carve(tg_svgf* s)
         s->guide[0] = s->guide[1] = s->hist[0] = s->hist[1] = s->tc = nullptr;
         s->grad = nullptr;
         s->fb_flags = nullptr;
-        s->d_err = static_cast<int*>(take(sizeof(int)));
+        s->d_err = static_cast<int*>(take(2 * sizeof(int)));
     } else {
         for (int k = 0; k < 2; ++k) {
             s->guide[k] = take(n * l.guide);
@@ -331,7 +331,7 @@ void carve(tg_svgf* s)
         s->colB = take(col_bytes_of(s->p, s->w, s->h));
         s->grad = static_cast<float2*>(take(n * sizeof(float2)));
         s->fb_flags = static_cast<int*>(take(fb_flags_bytes_of(s->w, s->h)));
-        s->d_err = static_cast<int*>(take(sizeof(int)));
+        s->d_err = static_cast<int*>(take(2 * sizeof(int)));
     }
 }
 
@@ -661,6 +661,7 @@ int launch_frame(tg_svgf* s, const tg_svgf_inputs* in, const tg_svgf_outputs* ou
         a.tc = s->tc;
         a.grad = s->grad;
         a.fb_flags = s->fb_flags;
+        a.fb_count = s->d_err + 1;
         a.err = s->d_err;
         a.alpha = s->p.alpha;
         a.alpha_m = s->p.moments_alpha;
@@ -687,8 +688,8 @@ int launch_frame(tg_svgf* s, const tg_svgf_inputs* in, const tg_svgf_outputs* ou
         });
         // variance: the block flags; the flagged blocks' short-history pixels (data-dependent, not counted)
         launch(s, stream, F_FULL_VARIANCE, double(fb_flags_bytes_of(s->w, s->h)), [&] {
-            const int vg = variance_grid(int(grd.x * grd.y), s->sms);
-            launch_chain(f16 ? k_full_variance<ST_FP16> : k_full_variance<ST_FP32>, dim3(vg), blk, stream, a);
+            const int vg = variance_list_grid(int(grd.x * grd.y), s->sms);
+            launch_chain(f16 ? k_full_variance<ST_FP16> : k_full_variance<ST_FP32>, dim3(vg), dim3(kBlockX, kBlockY / kVarR), stream, a);
         });
         void* src = s->colA;
         void* oth = s->colB;

@@ -178,7 +178,7 @@ cudaError_t launch_stages(tg_svgf_batch* b, int k, cudaStream_t s)
         const char* tab = b->d_table[k];
         const int L = int(st) - 2;
         if (st < 2)
-            e = launch_chain(pixel_kernel(f16, int(st)), dim3(g[st]), dim3(kBlockX, kBlockY), s, tab, b->cap);
+            e = launch_chain(pixel_kernel(f16, int(st)), dim3(g[st]), pixel_block(int(st)), s, tab, b->cap);
         else if (!b->stage_maps[b->R == 1 ? 0 : 1].empty())
             e = launch_chain(level_tma_kernel(f16, b->R, L, b->p.levels), dim3(g[st]), dim3(kLvTX, kLvRows), s, tab, b->cap,
                              L, b->stage_maps[b->R == 1 ? 0 : 1][st - 2]);

@@ -150,8 +150,7 @@ __global__ void __launch_bounds__(kLvTX* kLvRows, 6) k_batch_step(const char* __
                     const int j = find_stream(pf, hd.n, it), local = it - pf[j];
                     const FullArgs& a = ent[j].fa;
                     const int tx = (a.w + kBlockX - 1) / kBlockX;
-                    full_variance_tile<ST>(a, (local % tx) * kBlockX + threadIdx.x, (local / tx) * kBlockY + threadIdx.y,
-                                           *reinterpret_cast<VarTile*>(&sm));
+                    full_variance_tile<ST, 1>(a, (local % tx) * kBlockX, (local / tx) * kBlockY, *reinterpret_cast<VarTile*>(&sm));
                 }
                 __syncthreads();  // vl is refilled by the next chunk
             }
@@ -199,10 +198,13 @@ __global__ void __launch_bounds__(kLvTX* kLvRows, 6) k_batch_step(const char* __
 // hardware schedules the blocks; each kernel keeps its own occupancy.
 
 
-// STAGE 0 (K1): one CTA per pixel block.  STAGE 1 (K2): one chunk of
-// kVarPerCta blocks per CTA (gridDim.x = variance_grid(items, SMs)).
+// STAGE 0 (K1): one CTA of 32 x 4 threads per pixel block.  STAGE 1 (K2): one
+// chunk of kVarPerCta blocks per CTA of 32 x (4 / kVarR) threads (gridDim.x =
+// variance_grid(items, SMs)).
+__host__ inline dim3 pixel_block(int stage) { return dim3(kBlockX, stage == 0 ? kBlockY : kBlockY / kVarR); }
+
 template <int ST, int STAGE>
-__global__ void __launch_bounds__(kBlockX* kBlockY) k_ms_pixel(const char* __restrict__ table, int cap)
+__global__ void __launch_bounds__(STAGE == 0 ? kBlockX * kBlockY : kBlockX * kBlockY / kVarR, STAGE == 0 ? 8 : kVarCtas) k_ms_pixel(const char* __restrict__ table, int cap)
 {
     pdl_begin();
     const BatchHeader* hd = reinterpret_cast<const BatchHeader*>(table);
@@ -233,7 +235,7 @@ __global__ void __launch_bounds__(kBlockX* kBlockY) k_ms_pixel(const char* __res
             const int j = find_stream(pf, n_str, it), local = it - pf[j];
             const FullArgs& a = ent[j].fa;
             const int tx = (a.w + kBlockX - 1) / kBlockX;
-            full_variance_tile<ST>(a, (local % tx) * kBlockX + threadIdx.x, (local / tx) * kBlockY + threadIdx.y, vt);
+            full_variance_tile<ST, kVarR>(a, (local % tx) * kBlockX, (local / tx) * kBlockY, vt);
         }
     }
 }

@@ -78,7 +78,10 @@ struct FullArgs {
     size_t var_off;         // byte offset of the variance plane in col_src / col_dst
     size_t ghalf;           // FP32 records: index of the guide half-plane (16-byte units)
     float2* grad;           // per-pixel depth gradient (written by the temporal kernel)
-    int* fb_flags;          // per 32x4 pixel block: 1 if a pixel needs the spatial variance fallback
+    // Blocks of 32x4 pixels with a pixel that needs the spatial variance fallback: with a counter, fb_flags lists
+    // their numbers (in any order) and *fb_count is how many; without one (streams of a batch), fb_flags[block] is 1.
+    int* fb_flags;
+    int* fb_count;
     int* err;               // device error word (bounded waits that gave up); may be null
     ResLayout lin, lout;    // scratch layouts of col_src and col_dst
     float alpha, alpha_m, sigma_l, sigma_n, sigma_z;
@@ -242,83 +245,124 @@ struct VarTile {
     float2 m[kVarTH * kVarTW];  // luminance mean, variance
 };
 
-// `t` (the pixel's temporal colour and length) and `gr` (its depth gradient)
-// are loaded by the caller before it stages the tile.
-template <int ST>
-__device__ __forceinline__ void full_variance_px(const FullArgs& a, int x, int y, int cell, const VarTile& vt, float4 t,
-                                                 float2 gr)
+// One thread estimates R vertically adjacent pixels (x, y) .. (x, y + R - 1), so a
+// staged cell is read once for up to R of them: the pass is bound by shared-memory
+// bandwidth and the special-function unit.  `cell` is the first pixel's cell,
+// need[k] whether pixel k takes the estimate, gr[k] its depth gradient.
+template <int ST, int R>
+__device__ __forceinline__ void full_variance_px(const FullArgs& a, int x, int y, int cell, const VarTile& vt,
+                                                 const bool (&need)[R], const float2 (&gr)[R])
 {
-    typedef Stor<ST> S;
-    const size_t i = size_t(y) * a.w + x;
-    const int len = int(t.w);
-    if (len >= a.fallback_frames) return;
-    const float2 mom = vt.m[cell];
-    const float4 g = vt.g[cell];
     // w = max(0, n.n')^sigma_n exp(-|dz| / (sigma_z |grad z . off| + eps_z)), as one ex2;
     // offsets (dx, dy) and (-dx, -dy) share the depth scale kz
-    const float A_ = a.sigma_z * gr.x * (1.0f / kLog2eF), B_ = a.sigma_z * gr.y * (1.0f / kLog2eF);
     const float ez = kEpsZ * (1.0f / kLog2eF);
-    float kz[25];
+    float kz[R][25], s0[R], s1[R], s2[R];
+    float4 g[R];
+    float2 mom[R];
 #pragma unroll
-    for (int q = 0; q < 25; ++q) {
-        // q enumerates the offsets with dy < 0, or dy == 0 and dx <= 0 (the centre is q = 24)
-        const int dy = q < 21 ? q / 7 - 3 : 0;
-        const int dx = q < 21 ? q % 7 - 3 : q - 24;
-        kz[q] = rcp_approx(fabsf(fmaf(float(dx), A_, float(dy) * B_)) + ez);
+    for (int k = 0; k < R; ++k) {
+        const float A_ = a.sigma_z * gr[k].x * (1.0f / kLog2eF), B_ = a.sigma_z * gr[k].y * (1.0f / kLog2eF);
+#pragma unroll
+        for (int q = 0; q < 25; ++q) {
+            // q enumerates the offsets with dy < 0, or dy == 0 and dx <= 0 (the centre is q = 24)
+            const int dy = q < 21 ? q / 7 - 3 : 0;
+            const int dx = q < 21 ? q % 7 - 3 : q - 24;
+            kz[k][q] = rcp_approx(fabsf(fmaf(float(dx), A_, float(dy) * B_)) + ez);
+        }
+        mom[k] = vt.m[cell + k * kVarTW];
+        g[k] = vt.g[cell + k * kVarTW];
+        s0[k] = s1[k] = s2[k] = 0.0f;
     }
-    float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f;
 #pragma unroll
-    for (int dy = -kVarHalo; dy <= kVarHalo; ++dy) {
+    for (int r = -kVarHalo; r <= kVarHalo + R - 1; ++r) {
 #pragma unroll
         for (int dx = -kVarHalo; dx <= kVarHalo; ++dx) {
-            const bool neg = dy < 0 || (dy == 0 && dx <= 0);
-            const int ex = neg ? dx : -dx, ey = neg ? dy : -dy;
-            const int q = ey < 0 ? (ey + 3) * 7 + (ex + 3) : 24 + ex;
-            const int c = cell + dy * kVarTW + dx;
-            const float4 n = vt.g[c];
-            const float d = fmaf(n.z, g.z, fmaf(n.y, g.y, n.x * g.x));
-            float e = -fabsf(n.w - g.w) * kz[q];
-            e = fmaf(a.sigma_n, lg2_approx(fmaxf(d, 0.0f)), e);
-            const float wgt = ex2_approx(e);
-            const float2 m = vt.m[c];
-            const float dm = m.x - mom.x;
-            s0 += wgt;
-            s1 = fmaf(wgt, dm, s1);
-            s2 = fmaf(wgt, fmaf(dm, dm, m.y), s2);
+            const float4 n = vt.g[cell + r * kVarTW + dx];
+            const float2 m = vt.m[cell + r * kVarTW + dx];
+#pragma unroll
+            for (int k = 0; k < R; ++k) {
+                const int dy = r - k;
+                if (dy < -kVarHalo || dy > kVarHalo) continue;
+                const bool neg = dy < 0 || (dy == 0 && dx <= 0);
+                const int ex = neg ? dx : -dx, ey = neg ? dy : -dy;
+                const int q = ey < 0 ? (ey + 3) * 7 + (ex + 3) : 24 + ex;
+                const float d = fmaf(n.z, g[k].z, fmaf(n.y, g[k].y, n.x * g[k].x));
+                float e = -fabsf(n.w - g[k].w) * kz[k][q];
+                e = fmaf(a.sigma_n, lg2_approx(fmaxf(d, 0.0f)), e);
+                const float wgt = ex2_approx(e);
+                const float dm = m.x - mom[k].x;
+                s0[k] += wgt;
+                s1[k] = fmaf(wgt, dm, s1[k]);
+                s2[k] = fmaf(wgt, fmaf(dm, dm, m.y), s2[k]);
+            }
         }
     }
-    float var = mom.y;
-    if (s0 > 0.0f) {
-        const float m1 = s1 / s0;
-        var = fmaxf(0.0f, s2 / s0 - m1 * m1);
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        if (!need[k]) continue;
+        float var = mom[k].y;
+        if (s0[k] > 0.0f) {
+            const float m1 = s1[k] / s0[k];
+            var = fmaxf(0.0f, s2[k] / s0[k] - m1 * m1);
+        }
+        Rec::st_var(a.col_dst, a.var_off, size_t(y + k) * a.w + x, var);
     }
-    Rec::st_var(a.col_dst, a.var_off, i, var);
+}
+
+__device__ __forceinline__ int pixel_blocks(const FullArgs& a)
+{
+    return ((a.w + kBlockX - 1) / kBlockX) * ((a.h + kBlockY - 1) / kBlockY);
 }
 
 // One kBlockX x kBlockY pixel block `blk` (row-major over the image's blocks)
-// of K1 and K2.  K1 records in fb_flags[blk] whether any pixel of the block
-// needs the spatial fallback; K2 skips the blocks that need none.  Every thread
-// of the CTA calls these (K1 synchronises the CTA).
+// of K1 and K2.  K1 records whether any pixel of the block needs the spatial
+// fallback; K2 runs only those blocks.  Every thread of the CTA calls these (K1
+// synchronises the CTA).
 template <int ST> __device__ __forceinline__ void full_temporal_block(const FullArgs& a, int blk, int x, int y)
 {
     const bool fb = (x < a.w && y < a.h) ? full_temporal_px<ST>(a, x, y) : false;
     const int any = __syncthreads_or(fb);
-    if (threadIdx.x == 0 && threadIdx.y == 0) a.fb_flags[blk] = any;
+    if (threadIdx.x == 0 && threadIdx.y == 0) {
+        if (!a.fb_count)
+            a.fb_flags[blk] = any;
+        else if (any) {
+            const int at = atomicAdd(a.fb_count, 1);
+            if (at < pixel_blocks(a)) a.fb_flags[at] = blk;  // (always, unless a frame's launches failed half-way)
+        }
+    }
 }
 
-// K2 on one flagged pixel block; (x, y) is this thread's pixel of the block.
-template <int ST> __device__ __forceinline__ void full_variance_tile(const FullArgs& a, int x, int y, VarTile& vt)
+// Pixels of a column per K2 thread: a CTA of 32 x (4 / R) threads takes a pixel
+// block.  Two need 168 instead of 294 shared-memory wavefronts per 32 pixels; the
+// persistent batch kernel, whose CTAs have 128 threads, takes one.  Measured at
+// 1920x1080 after a cut (every block): frame 451 -> 423 us; a 3840x2160 frame
+// with some of its blocks listed 1184 -> 1176 us (with two pixels per thread but
+// flags instead of the list, 1184-1195: a CTA's share of the flagged blocks was
+// uneven).  10, 11 and 16 CTAs per SM: 425, 431 and 430 us.
+constexpr int kVarR = 2;
+constexpr int kVarCtas = 12;
+
+// K2 on one flagged pixel block at (bx, by); threadIdx is the thread's place in it.
+template <int ST, int R> __device__ __forceinline__ void full_variance_tile(const FullArgs& a, int bx, int by, VarTile& vt)
 {
     typedef Stor<ST> S;
-    const int x0 = x - int(threadIdx.x) - kVarHalo, y0 = y - int(threadIdx.y) - kVarHalo;
+    const int x = bx + int(threadIdx.x), y = by + int(threadIdx.y) * R;
+    const int x0 = bx - kVarHalo, y0 = by - kVarHalo;
     const typename S::guide_t* gc = static_cast<const typename S::guide_t*>(a.guide_cur);
     const typename S::mom_t* mc = static_cast<const typename S::mom_t*>(a.mom_cur);
-    // this thread's own pixel inputs, loaded before the staging so that their latency overlaps it
-    const bool own = x < a.w && y < a.h;
-    const size_t i = own ? size_t(y) * a.w + x : 0;
-    const float4 t = own ? S::ld4(static_cast<const typename S::c4_t*>(a.tc), i) : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float2 gr = own ? a.grad[i] : make_float2(0.f, 0.f);
-    for (int k = threadIdx.y * kBlockX + threadIdx.x; k < kVarTH * kVarTW; k += kBlockX * kBlockY) {
+    // this thread's own pixels' inputs, loaded before the staging so that their latency overlaps it
+    bool need[R];
+    float2 gr[R];
+    bool any = false;
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        const bool own = x < a.w && y + k < a.h;
+        const size_t i = own ? size_t(y + k) * a.w + x : 0;
+        need[k] = own && int(S::ld4_w(static_cast<const typename S::c4_t*>(a.tc), i)) < a.fallback_frames;
+        gr[k] = own ? a.grad[i] : make_float2(0.f, 0.f);
+        any |= need[k];
+    }
+    for (int k = threadIdx.y * kBlockX + threadIdx.x; k < kVarTH * kVarTW; k += kBlockX * kBlockY / R) {
         const int qy = y0 + k / kVarTW, qx = x0 + k % kVarTW;
         float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
         float2 m = make_float2(0.f, 0.f);
@@ -331,11 +375,12 @@ template <int ST> __device__ __forceinline__ void full_variance_tile(const FullA
         vt.m[k] = m;
     }
     __syncthreads();
-    if (own) full_variance_px<ST>(a, x, y, (int(threadIdx.y) + kVarHalo) * kVarTW + int(threadIdx.x) + kVarHalo, vt, t, gr);
+    if (any)
+        full_variance_px<ST, R>(a, x, y, (int(threadIdx.y) * R + kVarHalo) * kVarTW + int(threadIdx.x) + kVarHalo, vt, need, gr);
     __syncthreads();  // the tile's storage is reused by the caller's next block
 }
 
-// K2 grids: a CTA takes the pixel blocks base + t * stride (t < kVarPerCta) of
+// K2 grids over flags (batches): a CTA takes the pixel blocks base + t * stride (t < kVarPerCta) of
 // its chunk, compacts the flagged ones into a shared list and runs only those,
 // so that the mostly unflagged blocks of a frame cost one parallel flag read
 // per chunk instead of one CTA each.
@@ -343,7 +388,7 @@ constexpr int kVarPerCta = 32;
 
 __host__ __device__ inline int variance_grid(int items, int sms)
 {
-    const int lo = (items + kVarPerCta - 1) / kVarPerCta, hi = items < 6 * sms ? items : 6 * sms;
+    const int lo = (items + kVarPerCta - 1) / kVarPerCta, hi = items < 12 * sms ? items : 12 * sms;
     return lo > hi ? lo : hi;
 }
 
@@ -374,20 +419,19 @@ template <int ST> __global__ void __launch_bounds__(kBlockX* kBlockY, 8) k_full_
                             blockIdx.y * kBlockY + threadIdx.y);
 }
 
-// One chunk per CTA: gridDim.x = variance_grid(blocks, SMs) covers every block.
-template <int ST> __global__ void __launch_bounds__(kBlockX* kBlockY) k_full_variance(FullArgs a)
+// The listed blocks, one at a time per CTA of one resident wave (kVarCtas per SM).
+// Level 0 clears the counter for the next frame.
+template <int ST> __global__ void __launch_bounds__(kBlockX* kBlockY / kVarR, kVarCtas) k_full_variance(FullArgs a)
 {
     __shared__ VarTile vt;
-    __shared__ VarList l;
     pdl_begin();
-    const int tx = (a.w + kBlockX - 1) / kBlockX, items = tx * ((a.h + kBlockY - 1) / kBlockY);
-    const int* flags = a.fb_flags;
-    variance_compact(int(blockIdx.x), int(gridDim.x), items, [flags](int b) { return __ldcg(flags + b) != 0; }, l);
-    const int n = l.n;
-    for (int e = 0; e < n; ++e) {
-        const int b = l.item[e];
-        full_variance_tile<ST>(a, (b % tx) * kBlockX + threadIdx.x, (b / tx) * kBlockY + threadIdx.y, vt);
+    const int tx = (a.w + kBlockX - 1) / kBlockX, n = min(__ldcg(a.fb_count), pixel_blocks(a));
+    for (int e = blockIdx.x; e < n; e += gridDim.x) {
+        const int b = __ldcg(a.fb_flags + e);
+        full_variance_tile<ST, kVarR>(a, (b % tx) * kBlockX, (b / tx) * kBlockY, vt);
     }
 }
+
+__host__ inline int variance_list_grid(int blocks, int sms) { return blocks < kVarCtas * sms ? blocks : kVarCtas * sms; }
 
 } // namespace tg

@@ -388,6 +388,12 @@ __device__ __forceinline__ void plane_cell(const FullArgs& a, const LevelArgs& l
     }
 }
 
+// K2 has read the list of fallback blocks; the next frame's K1 starts an empty one.
+__device__ __forceinline__ void clear_fallback_count(const FullArgs& a)
+{
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0 && a.fb_count) *a.fb_count = 0;
+}
+
 // One tile of one level, staged with plain coalesced loads (the residue-major
 // records of a tile row are contiguous; PL: level 0 from the planes).  The
 // caller synchronises the CTA before reusing `sm`.
@@ -437,6 +443,7 @@ __global__ void __launch_bounds__(kLvTX* kLvRows, LevelOcc<R>::kCtas) k_full_lev
 {
     __shared__ LevelSmem<R> sm;
     pdl_begin();
+    if (PL) clear_fallback_count(a);
     full_level_tile<ST, R, VAR, PL>(a, level_args_of(a), g, tile_of_grid<R>(g), sm);
 }
 
@@ -643,6 +650,7 @@ __global__ void __launch_bounds__(kLvTX* kLvRows, LevelOcc<R>::kCtas)
     __shared__ LevelSmem<R> sm;
     __shared__ __align__(8) uint64_t bar;
     pdl_begin();
+    if (PL) clear_fallback_count(a);
     full_level_tile_tma<ST, R, VAR, PL>(a, lv, g, tile_of_grid<R>(g), sm, bar, &tm, &tm2);
 }
 

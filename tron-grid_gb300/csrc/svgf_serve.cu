@@ -175,6 +175,7 @@ struct tg_svgf_server {
     char* h_table[kMaxInflight] = {};
     int* h_err = nullptr;
     BarrierState* d_bar = nullptr;
+    int* d_fb = nullptr;  // counter of fallback blocks of the plain path
     cudaGraphExec_t exec[kMaxInflight] = {};
     std::vector<cudaEvent_t> ev_pool;  // completion events, reused
     StageMaps stage_maps[10];          // the stage kernels' maps of the launch being formed (one per level)
@@ -356,7 +357,7 @@ void launch_stage_kernels(tg_svgf_server* sv, int k, const std::vector<int>& gri
         if (g < 2) {
             auto p16 = g == 0 ? k_ms_pixel<ST_FP16, 0> : k_ms_pixel<ST_FP16, 1>;
             auto p32 = g == 0 ? k_ms_pixel<ST_FP32, 0> : k_ms_pixel<ST_FP32, 1>;
-            launch_chain(sv->f16 ? p16 : p32, dim3(grids[g]), dim3(kBlockX, kBlockY), st, tab, sv->cap);
+            launch_chain(sv->f16 ? p16 : p32, dim3(grids[g]), pixel_block(int(g)), st, tab, sv->cap);
         } else {
             // level 0 stages from the planes, the last level writes only colour
             const int L = int(g) - 2;
@@ -449,9 +450,10 @@ void launch_plain(tg_svgf_server* sv, Sess& s)
     const dim3 blk(kBlockX, kBlockY);
     const dim3 grd((s.w + kBlockX - 1) / kBlockX, (s.h + kBlockY - 1) / kBlockY);
     cudaStream_t st = sv->s_comp;
-    const int vg = variance_grid(int(grd.x * grd.y), sv->sm_count);
+    a.fb_count = sv->d_fb;  // (launches are ordered on s_comp)
+    const int vg = variance_list_grid(int(grd.x * grd.y), sv->sm_count);
     launch_chain(sv->f16 ? k_full_temporal<ST_FP16> : k_full_temporal<ST_FP32>, grd, blk, st, a);
-    launch_chain(sv->f16 ? k_full_variance<ST_FP16> : k_full_variance<ST_FP32>, dim3(vg), blk, st, a);
+    launch_chain(sv->f16 ? k_full_variance<ST_FP16> : k_full_variance<ST_FP32>, dim3(vg), dim3(kBlockX, kBlockY / kVarR), st, a);
     void* src = s.colA;
     void* oth = s.colB;
     for (int lv = 0; lv < sv->d.params.levels; ++lv) {
@@ -747,6 +749,7 @@ void teardown(tg_svgf_server* sv)
     for (cudaEvent_t e : sv->ev_pool) cudaEventDestroy(e);
     if (sv->h_err) cudaFreeHost(sv->h_err);
     if (sv->d_bar) cudaFree(sv->d_bar);
+    if (sv->d_fb) cudaFree(sv->d_fb);
     if (sv->base) cudaFree(sv->base);
     cudaStream_t streams[4] = {sv->s_h2d, sv->s_comp, sv->s_d2h, sv->cap_stream};
     for (auto s : streams)
@@ -818,9 +821,13 @@ int tg_svgf_server_create(const tg_svgf_server_desc* d, tg_svgf_server** out)
                 return bail(fail(TG_ERR_OOM, "work table allocation failed"));
         if (cudaHostAlloc(reinterpret_cast<void**>(&sv->h_err), kMaxInflight * sizeof(int), cudaHostAllocDefault) !=
                 cudaSuccess ||
-            cudaMalloc(&sv->d_bar, sizeof(BarrierState)) != cudaSuccess)
+            cudaMalloc(&sv->d_bar, sizeof(BarrierState) + sizeof(int)) != cudaSuccess)
             return bail(fail(TG_ERR_OOM, "barrier allocation failed"));
         for (int k = 0; k < kMaxInflight; ++k) sv->h_err[k] = 0;
+    }
+    if (cudaMalloc(&sv->d_fb, sizeof(int)) != cudaSuccess || cudaMemset(sv->d_fb, 0, sizeof(int)) != cudaSuccess) {
+        cudaGetLastError();
+        return bail(fail(TG_ERR_OOM, "fallback counter allocation failed"));
     }
     if (cudaDeviceSynchronize() != cudaSuccess) return bail(fail(TG_ERR_CUDA, "server initialisation failed"));
     try {
