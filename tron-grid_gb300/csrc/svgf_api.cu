@@ -208,6 +208,7 @@ template <int ST, int R> LevelTmaFn level_tma_kernel_r(bool pl, bool last)
 LevelTmaFn level_tma_kernel(bool f16, bool pl, bool last, int rows)
 {
     if (rows == 3) return f16 ? level_tma_kernel_r<ST_FP16, 3>(pl, last) : level_tma_kernel_r<ST_FP32, 3>(pl, last);
+    if (rows == 1) return f16 ? level_tma_kernel_r<ST_FP16, 1>(pl, last) : level_tma_kernel_r<ST_FP32, 1>(pl, last);
     // (two rows: never the last level, level_rows)
     if (f16) return pl ? k_full_level_tma<ST_FP16, 2, true, true> : k_full_level_tma<ST_FP16, 2, true, false>;
     return pl ? k_full_level_tma<ST_FP32, 2, true, true> : k_full_level_tma<ST_FP32, 2, true, false>;
@@ -427,7 +428,7 @@ void build_tensor_maps(tg_svgf* s)
         s->tma = true;  // interior tiles of the later passes (where their planes allow) and of the first pass
         return;
     }
-    for (int R = 2; R <= 3; ++R) {
+    for (int R = 1; R <= 3; ++R) {
         CUtensorMap maps[kFullMaps];
         const unsigned m = full_level_maps(s->p, s->w, s->h, R, s->colA, s->colB, s->tc, s->guide[0], s->guide[1], maps);
         for (int lv = 1; lv < s->p.levels; ++lv) {
