@@ -207,6 +207,13 @@ def load(path: str = LIB_PATH):
     return lib
 
 
+def packed(name: str):
+    """Entry point (handle, inputs, outputs, stream) that takes its structures as packed bytes."""
+    fn = load()[name]  # a function object of its own
+    fn.restype, fn.argtypes = C.c_int, [_P, C.c_char_p, C.c_char_p, _P]
+    return fn
+
+
 def check(status: int):
     if status != OK:
         msg = load().tg_last_error()

@@ -8,15 +8,12 @@ float32 depth in CPU-visible memory, triple-buffered, read two frames behind).
 from __future__ import annotations
 
 import ctypes as C
+import struct
 
 import numpy as np
 import torch
 
 from . import _lib as L
-
-
-def _image(t, fmt):
-    return L.Image(t.data_ptr(), t.stride(0) * t.element_size(), fmt, 0)
 
 
 def colour_format(t, order="bgra"):
@@ -50,6 +47,11 @@ class EyeReadback:
         h = C.c_void_p()
         L.check(self.lib.tg_eye_create(C.byref(d), C.byref(h)))
         self.handle = h
+        self._submit = self.lib["tg_eye_submit"]  # a function object of its own: images as packed bytes
+        self._submit.restype, self._submit.argtypes = C.c_int, [C.c_void_p, C.c_uint64, C.c_char_p, C.c_char_p, C.c_void_p]
+        self._images = struct.Struct("Qqii" * self.n)
+        assert self._images.size == self.n * C.sizeof(L.Image)
+        self._views = {}  # ring slot -> the eyes' views of it (a slot's memory stays where it is)
 
     def host_bytes(self) -> int:
         return int(self.lib.tg_eye_host_bytes(self.n, self._w, self._h, self.ring))
@@ -58,21 +60,25 @@ class EyeReadback:
         """colours: per eye (h, w, 4) uint8 / float16 / float32 CUDA tensors; depths: per eye (h, w) float32."""
         if len(colours) != self.n or len(depths) != self.n:
             raise ValueError(f"{self.n} eyes, {len(colours)} colour and {len(depths)} depth images given")
-        ci = (L.Image * self.n)(*[_image(c, colour_format(c, order)) for c in colours])
-        di = (L.Image * self.n)(*[_image(d, L.FMT_R32F) for d in depths])
+        ci, di = [], []
+        for c in colours:
+            ci += (c.data_ptr(), c.stride(0) * c.element_size(), colour_format(c, order), 0)
+        for d in depths:
+            di += (d.data_ptr(), d.stride(0) * d.element_size(), L.FMT_R32F, 0)
         s = stream if stream is not None else torch.cuda.current_stream(self.device)
-        L.check(self.lib.tg_eye_submit(self.handle, frame, ci, di, C.c_void_p(s.cuda_stream)))
+        L.check(self._submit(self.handle, frame, self._images.pack(*ci), self._images.pack(*di), s.cuda_stream))
 
     def acquire(self, frame: int):
         """[(rgb (h, w, 3) uint8, depth (h, w) float32, fov)] views into the host slot of `frame`."""
         out = (L.VisionData * self.n)()
         L.check(self.lib.tg_eye_acquire(self.handle, frame, out))
-        res = []
-        for v in out:
-            rgb = np.ctypeslib.as_array(v.rgb, shape=(v.height, v.width, 3))
-            dep = np.ctypeslib.as_array(v.depth, shape=(v.height, v.width))
-            res.append((rgb, dep, v.fov_horizontal))
-        return res
+        slot = frame % (self.ring or 3)  # (0: the library's default ring of 3)
+        views = self._views.get(slot)
+        if views is None:
+            views = self._views[slot] = [
+                (np.ctypeslib.as_array(v.rgb, shape=(v.height, v.width, 3)),
+                 np.ctypeslib.as_array(v.depth, shape=(v.height, v.width)), v.fov_horizontal) for v in out]
+        return [(rgb[:], dep[:], fov) for rgb, dep, fov in views]
 
     def close(self):
         if self.handle:
