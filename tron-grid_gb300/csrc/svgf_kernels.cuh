@@ -77,7 +77,7 @@ struct FullArgs {
     void* col_dst;
     size_t var_off;         // byte offset of the variance plane in col_src / col_dst
     size_t ghalf;           // FP32 records: index of the guide half-plane (16-byte units)
-    float2* grad;           // per-pixel depth gradient (written by the temporal kernel)
+    float2* grad;           // per-pixel depth gradient (written by the temporal kernel), at grad_idx
     // Blocks of 32x4 pixels with a pixel that needs the spatial variance fallback: with a counter, fb_flags lists
     // their numbers (in any order) and *fb_count is how many; without one (streams of a batch), fb_flags[block] is 1.
     int* fb_flags;
@@ -89,6 +89,16 @@ struct FullArgs {
     int max_history, fallback_frames;
     int level, stride, last;
 };
+
+// Where the depth gradient of column x lies in its row: the four residues of x
+// mod 4 one after the other.  A warp of a level reads every s-th column, which
+// touches 2, 4, 8, 16, 32 cache lines of row-major gradients at strides 1 to 16,
+// and 4, 2, 2, 4, 8 of these.
+__device__ __forceinline__ int grad_col(int w, int x)
+{
+    const int r = x & 3;
+    return r * (w >> 2) + min(r, w & 3) + (x >> 2);
+}
 
 // K1: guide write, reprojection (bilinear 2x2 with depth/normal test), history
 // length, colour EMA and mean-centred moment EMA.  A pixel whose history is at
@@ -163,7 +173,7 @@ template <int ST> __device__ __forceinline__ bool full_temporal_px(const FullArg
     static_cast<G*>(a.guide_cur)[i] = gv;
     const float gx = grad1(z, zl, zr, hl, hr);
     const float gy = grad1(z, zu, zd, hu, hd);
-    a.grad[i] = make_float2(gx, gy);
+    a.grad[size_t(y) * a.w + grad_col(a.w, x)] = make_float2(gx, gy);
     const float cr = S::qin(c4.x), cg = S::qin(c4.y), cb = S::qin(c4.z);
     const float gsum = __fadd_rn(fabsf(gx), fabsf(gy));
     const float ztol = __fadd_rn(__fadd_rn(__fmul_rn(kDepthRel, z), __fmul_rn(kDepthGrad, gsum)), kDepthAbs);
@@ -359,7 +369,7 @@ template <int ST, int R> __device__ __forceinline__ void full_variance_tile(cons
         const bool own = x < a.w && y + k < a.h;
         const size_t i = own ? size_t(y + k) * a.w + x : 0;
         need[k] = own && int(S::ld4_w(static_cast<const typename S::c4_t*>(a.tc), i)) < a.fallback_frames;
-        gr[k] = own ? a.grad[i] : make_float2(0.f, 0.f);
+        gr[k] = own ? a.grad[size_t(y + k) * a.w + grad_col(a.w, x)] : make_float2(0.f, 0.f);
         any |= need[k];
     }
     for (int k = threadIdx.y * kBlockX + threadIdx.x; k < kVarTH * kVarTW; k += kBlockX * kBlockY / R) {

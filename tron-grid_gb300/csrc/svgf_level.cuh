@@ -193,7 +193,7 @@ __device__ __forceinline__ void level_prefetch(const FullArgs& a, const LevelArg
 {
     typedef Stor<ST> S;
     const int lg = lv.lin.lg, m = s - 1, pw = lv.lin.pw, P = lv.lin.pw * lv.lin.ph;
-    const int cx = ra + s * (i0 + int(threadIdx.x));
+    const int cx = ra + s * (i0 + int(threadIdx.x)), gx = grad_col(a.w, cx);
     int cxo[3];
     bool cxv[3];
 #pragma unroll
@@ -217,7 +217,7 @@ __device__ __forceinline__ void level_prefetch(const FullArgs& a, const LevelArg
     for (int k = 0; k < R; ++k) {
         const int y = rb + s * (j0 + int(threadIdx.y) * R + k);
         pre.valid[k] = IN || (cx < a.w && y < a.h);
-        pre.gr[k] = pre.valid[k] ? a.grad[y * a.w + cx] : make_float2(0.f, 0.f);
+        pre.gr[k] = pre.valid[k] ? a.grad[y * a.w + gx] : make_float2(0.f, 0.f);
 #pragma unroll
         for (int f = 0; f < 3; ++f) {
             const bool oy = pre.valid[k] && (IN || unsigned(y + f - 1) < unsigned(a.h));
