@@ -124,7 +124,7 @@ template <int ST> __device__ __forceinline__ bool full_temporal_px(const FullArg
     const float2 mv = ld_motion(a.motion, x, y);
     const float4 c4 = ld_rgba(a.radiance, x, y);
     uint32_t enc = 0;
-    float3 n = ld_normal(a.normal, x, y, ST == ST_FP16, enc);
+    const float3 n = ld_normal(a.normal, x, y, ST == ST_FP16, enc);
     const float z = ld_depth(a.depth, x, y);
     const bool hl = x > 0, hr = x < a.w - 1, hu = y > 0, hd = y < a.h - 1;
     const float zl = hl ? ld_depth(a.depth, x - 1, y) : 0.0f, zr = hr ? ld_depth(a.depth, x + 1, y) : 0.0f;
@@ -153,22 +153,22 @@ template <int ST> __device__ __forceinline__ bool full_temporal_px(const FullArg
         tin[k] = tx >= 0 && ty >= 0 && tx < a.w && ty < a.h;
         tj[k] = tin[k] ? size_t(ty) * a.w + tx : 0;
     }
-    float4 thv[4], tg[4];
+    float4 thv[4];
+    typename S::graw_t tg[4];
     float2 tm[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         if (tin[k]) {
             thv[k] = S::ld4(hp, tj[k]);
-            tg[k] = S::ld_guide_raw(gp, tj[k]);
+            tg[k] = S::ld_graw(gp, tj[k]);
             tm[k] = S::ldm(mp, tj[k]);
         } else {
             thv[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-            tg[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            tg[k] = typename S::graw_t{};
             tm[k] = make_float2(0.f, 0.f);
         }
     }
 
-    if (ST == ST_FP16) n = oct16_decode_raw(enc);  // FP16 storage keeps the octahedral code
     const G gv = S::mk_guide(n, enc, z);
     static_cast<G*>(a.guide_cur)[i] = gv;
     const float gx = grad1(z, zl, zr, hl, hr);
@@ -176,6 +176,10 @@ template <int ST> __device__ __forceinline__ bool full_temporal_px(const FullArg
     a.grad[size_t(y) * a.w + grad_col(a.w, x)] = make_float2(gx, gy);
     const float cr = S::qin(c4.x), cg = S::qin(c4.y), cb = S::qin(c4.z);
     const float gsum = __fadd_rn(fabsf(gx), fabsf(gy));
+    bool other = false;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) other |= tin[k] && !S::same_normal(tg[k], gv);
+    const float3 nt = S::test_normal(gv, other);
     const float ztol = __fadd_rn(__fadd_rn(__fmul_rn(kDepthRel, z), __fmul_rn(kDepthGrad, gsum)), kDepthAbs);
     float sw = 0.0f, hr_ = 0.0f, hg = 0.0f, hb = 0.0f, hmu = 0.0f;
     float tw[4];
@@ -184,8 +188,8 @@ template <int ST> __device__ __forceinline__ bool full_temporal_px(const FullArg
     for (int k = 0; k < 4; ++k) {
         tw[k] = 0.0f;
         if (!tin[k] || !(thv[k].w > 0.0f)) continue;
-        if (!(fabsf(__fsub_rn(tg[k].w, z)) <= ztol)) continue;
-        if (!normal_close(tg[k].x, tg[k].y, tg[k].z, n.x, n.y, n.z)) continue;
+        if (!(fabsf(__fsub_rn(S::graw_z(tg[k]), z)) <= ztol)) continue;
+        if (!S::normal_close_to(tg[k], gv, nt)) continue;
         tw[k] = bw[k];
         sw = __fadd_rn(sw, bw[k]);
         hr_ += bw[k] * thv[k].x;
