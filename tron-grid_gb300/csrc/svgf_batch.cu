@@ -130,9 +130,9 @@ int set_config(tg_svgf_batch* b, int strategy, int R, int ctas)
     return TG_OK;
 }
 
-using PixFn = void (*)(const char*, int);
-using LevFn = void (*)(const char*, int, int);
-using LevTmaFn = void (*)(const char*, int, int, const StageMaps);
+using PixFn = void (*)(const char*, int, const BatchParams);
+using LevFn = void (*)(const char*, int, int, const BatchParams);
+using LevTmaFn = void (*)(const char*, int, int, const BatchParams, const StageMaps);
 
 PixFn pixel_kernel(bool f16, int stage)
 {
@@ -173,17 +173,18 @@ cudaError_t launch_stages(tg_svgf_batch* b, int k, cudaStream_t s)
         return e;
     const bool f16 = b->p.storage == TG_SVGF_STORAGE_FP16;
     const std::vector<int>& g = b->grids[k];
+    const BatchParams bp = batch_params(b->p, sigma_n_squarings(b->p.sigma_n));
     for (size_t st = 0; st < g.size(); ++st) {
         if (g[st] <= 0) continue;
         const char* tab = b->d_table[k];
         const int L = int(st) - 2;
         if (st < 2)
-            e = launch_chain(pixel_kernel(f16, int(st)), dim3(g[st]), pixel_block(int(st)), s, tab, b->cap);
+            e = launch_chain(pixel_kernel(f16, int(st)), dim3(g[st]), pixel_block(int(st)), s, tab, b->cap, bp);
         else if (!b->stage_maps[b->R == 1 ? 0 : 1].empty())
             e = launch_chain(level_tma_kernel(f16, b->R, L, b->p.levels), dim3(g[st]), dim3(kLvTX, kLvRows), s, tab, b->cap,
-                             L, b->stage_maps[b->R == 1 ? 0 : 1][st - 2]);
+                             L, bp, b->stage_maps[b->R == 1 ? 0 : 1][st - 2]);
         else
-            e = launch_chain(level_kernel(f16, b->R, L, b->p.levels), dim3(g[st]), dim3(kLvTX, kLvRows), s, tab, b->cap, L);
+            e = launch_chain(level_kernel(f16, b->R, L, b->p.levels), dim3(g[st]), dim3(kLvTX, kLvRows), s, tab, b->cap, L, bp);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;

@@ -56,7 +56,7 @@ constexpr int kTmaStreams = 80;
 struct StageMaps {
     CUtensorMap m[3 * kTmaStreams];
 };
-static_assert(sizeof(StageMaps) + 64 <= 32764, "stage maps must fit the kernel parameter space");
+static_assert(sizeof(StageMaps) + 192 <= 32764, "stage maps must fit the kernel parameter space");
 
 constexpr int kStages = 2 + 10;
 constexpr long long kBarrierSpinCycles = 2000000000LL;  // default limit, ~1 s at 2 GHz
@@ -114,6 +114,47 @@ __device__ __forceinline__ int find_stream(const int* pf, int n, int item)
             hi = mid;
     }
     return lo;
+}
+
+// The same by a whole warp (32 lanes of a row, one item): as many prefixes as are
+// at most the item.  One load per 32 streams instead of a chain of them.
+__device__ __forceinline__ int find_stream_warp(const int* pf, int n, int item)
+{
+    if (n > 256) return find_stream(pf, n, item);
+    int c = 0;
+    for (int i = 0; i < n; i += 32) {
+        const int k = i + int(threadIdx.x);
+        c += __popc(__ballot_sync(0xffffffffu, k < n && pf[k] <= item));
+    }
+    return c - 1;
+}
+
+// The parameters all streams share, which the stage kernels take as a kernel
+// parameter: a constant operand then, where an entry's field is a load and a
+// register.
+struct BatchParams {
+    float alpha, alpha_m, sigma_l, sigma_n, sigma_z;
+    int sq_n, max_history, fallback_frames, levels;
+};
+
+inline BatchParams batch_params(const tg_svgf_params& p, int sq_n)
+{
+    return {p.alpha, p.moments_alpha, p.sigma_l, p.sigma_n, p.sigma_z, sq_n, p.max_history, p.fallback_frames, p.levels};
+}
+
+__device__ __forceinline__ FullArgs stream_args(const BatchEntry& e, const BatchParams& c)
+{
+    FullArgs a = e.fa;
+    a.fb_count = nullptr;
+    a.alpha = c.alpha;
+    a.alpha_m = c.alpha_m;
+    a.sigma_l = c.sigma_l;
+    a.sigma_n = c.sigma_n;
+    a.sigma_z = c.sigma_z;
+    a.sq_n = c.sq_n;
+    a.max_history = c.max_history;
+    a.fallback_frames = c.fallback_frames;
+    return a;
 }
 
 // The persistent kernel runs the pixel stages on its level-shaped CTAs, and
@@ -177,7 +218,7 @@ __global__ void __launch_bounds__(kLvTX* kLvRows, 6) k_batch_step(const char* __
                 lv.last = L == hd.levels - 1;
                 lv.lin = res_layout(a.w, a.h, L);
                 lv.lout = res_layout(a.w, a.h, L + 1);
-                const LevelGeom g = level_geom(a.w, a.h, 1 << L, R);
+                const LevelGeom g = level_geom_lg(a.w, a.h, L, R);
                 // level 0 stages from the planes; the last level writes only colour
                 if (L == 0)
                     full_level_tile<ST, R, true, true>(a, lv, g, tile_of_id<R>(g, local), sm);
@@ -204,7 +245,7 @@ __global__ void __launch_bounds__(kLvTX* kLvRows, 6) k_batch_step(const char* __
 __host__ inline dim3 pixel_block(int stage) { return dim3(kBlockX, stage == 0 ? kBlockY : kBlockY / kVarR); }
 
 template <int ST, int STAGE>
-__global__ void __launch_bounds__(STAGE == 0 ? kBlockX * kBlockY : kBlockX * kBlockY / kVarR, STAGE == 0 ? 8 : kVarCtas) k_ms_pixel(const char* __restrict__ table, int cap)
+__global__ void __launch_bounds__(STAGE == 0 ? kBlockX * kBlockY : kBlockX * kBlockY / kVarR, STAGE == 0 ? 8 : kVarCtas) k_ms_pixel(const char* __restrict__ table, int cap, const BatchParams c)
 {
     pdl_begin();
     const BatchHeader* hd = reinterpret_cast<const BatchHeader*>(table);
@@ -214,9 +255,9 @@ __global__ void __launch_bounds__(STAGE == 0 ? kBlockX * kBlockY : kBlockX * kBl
     if constexpr (STAGE == 0) {
         const int item = blockIdx.x;
         if (item >= items) return;
-        const int j = find_stream(pf, n_str, item);
+        const int j = find_stream_warp(pf, n_str, item);
         const int local = item - pf[j];
-        const FullArgs& a = ent[j].fa;
+        const FullArgs& a = ent[j].fa;  // (with c's constants the blend contracts differently from the single stream's)
         const int tx = (a.w + kBlockX - 1) / kBlockX;
         full_temporal_block<ST>(a, local, (local % tx) * kBlockX + threadIdx.x, (local / tx) * kBlockY + threadIdx.y);
     } else {
@@ -233,7 +274,7 @@ __global__ void __launch_bounds__(STAGE == 0 ? kBlockX * kBlockY : kBlockX * kBl
         for (int e = 0; e < n; ++e) {
             const int it = vl.item[e];
             const int j = find_stream(pf, n_str, it), local = it - pf[j];
-            const FullArgs& a = ent[j].fa;
+            const FullArgs a = stream_args(ent[j], c);
             const int tx = (a.w + kBlockX - 1) / kBlockX;
             full_variance_tile<ST, kVarR>(a, (local % tx) * kBlockX, (local / tx) * kBlockY, vt);
         }
@@ -242,7 +283,7 @@ __global__ void __launch_bounds__(STAGE == 0 ? kBlockX * kBlockY : kBlockX * kBl
 
 // VAR = false at the last level (colour only); PL at level 0 (staged from the planes).
 template <int ST, int R, bool VAR, bool PL>
-__global__ void __launch_bounds__(kLvTX* kLvRows, LevelOcc<R>::kCtas) k_ms_level(const char* __restrict__ table, int cap, int L)
+__global__ void __launch_bounds__(kLvTX* kLvRows, LevelOcc<R>::kCtas) k_ms_level(const char* __restrict__ table, int cap, int L, const BatchParams c)
 {
     __shared__ LevelSmem<R> sm;
     pdl_begin();
@@ -250,19 +291,19 @@ __global__ void __launch_bounds__(kLvTX* kLvRows, LevelOcc<R>::kCtas) k_ms_level
     const int* pf = reinterpret_cast<const int*>(table + table_prefix_offset()) + (2 + L) * (cap + 1);
     const int item = blockIdx.x;
     if (item >= pf[hd->n]) return;
-    const int j = find_stream(pf, hd->n, item);
+    const int j = find_stream_warp(pf, hd->n, item);
     const BatchEntry& e = reinterpret_cast<const BatchEntry*>(table + table_entries_offset(cap))[j];
-    const FullArgs& a = e.fa;
+    const FullArgs a = stream_args(e, c);
     LevelArgs lv;
     lv.col_src = (L & 1) ? e.colB : e.colA;
     lv.col_dst = (L & 1) ? e.colA : e.colB;
     lv.var_off = a.var_off;
     lv.ghalf = a.ghalf;
     lv.level = L;
-    lv.last = L == hd->levels - 1;
+    lv.last = L == c.levels - 1;
     lv.lin = res_layout(a.w, a.h, L);
     lv.lout = res_layout(a.w, a.h, L + 1);
-    const LevelGeom g = level_geom(a.w, a.h, 1 << L, R);
+    const LevelGeom g = level_geom_lg(a.w, a.h, L, R);
     full_level_tile<ST, R, VAR, PL>(a, lv, g, tile_of_id<R>(g, item - pf[j]), sm);
 }
 
@@ -271,7 +312,7 @@ __global__ void __launch_bounds__(kLvTX* kLvRows, LevelOcc<R>::kCtas) k_ms_level
 // otherwise.
 template <int ST, int R, bool VAR, bool PL>
 __global__ void __launch_bounds__(kLvTX* kLvRows, LevelOcc<R>::kCtas)
-    k_ms_level_tma(const char* __restrict__ table, int cap, int L, const __grid_constant__ StageMaps maps)
+    k_ms_level_tma(const char* __restrict__ table, int cap, int L, const BatchParams c, const __grid_constant__ StageMaps maps)
 {
     __shared__ LevelSmem<R> sm;
     __shared__ __align__(8) uint64_t bar;
@@ -280,19 +321,19 @@ __global__ void __launch_bounds__(kLvTX* kLvRows, LevelOcc<R>::kCtas)
     const int* pf = reinterpret_cast<const int*>(table + table_prefix_offset()) + (2 + L) * (cap + 1);
     const int item = blockIdx.x;
     if (item >= pf[hd->n]) return;
-    const int j = find_stream(pf, hd->n, item);
+    const int j = find_stream_warp(pf, hd->n, item);
     const BatchEntry& e = reinterpret_cast<const BatchEntry*>(table + table_entries_offset(cap))[j];
-    const FullArgs& a = e.fa;
+    const FullArgs a = stream_args(e, c);
     LevelArgs lv;
     lv.col_src = (L & 1) ? e.colB : e.colA;
     lv.col_dst = (L & 1) ? e.colA : e.colB;
     lv.var_off = a.var_off;
     lv.ghalf = a.ghalf;
     lv.level = L;
-    lv.last = L == hd->levels - 1;
+    lv.last = L == c.levels - 1;
     lv.lin = res_layout(a.w, a.h, L);
     lv.lout = res_layout(a.w, a.h, L + 1);
-    const LevelGeom g = level_geom(a.w, a.h, 1 << L, R);
+    const LevelGeom g = level_geom_lg(a.w, a.h, L, R);
     if (e.tma_slot >= 0 && ((e.tma_mask >> L) & 1u)) {
         // level 0 stages from the tc plane and this step's guide plane, the others from their records
         const CUtensorMap* tm = PL ? &maps.m[3 * e.tma_slot] : &maps.m[e.tma_slot];

@@ -113,9 +113,18 @@ __device__ __forceinline__ void level_block(const LevelGeom& g, int bid, int TX,
     const unsigned tile = u >> (2 * g.lg);
     ra = int(res & unsigned(g.s - 1));
     rb = int(res >> g.lg);
-    const unsigned ty = tile / unsigned(g.tiles_x);
-    i0 = int(tile - ty * unsigned(g.tiles_x)) * TX;
-    j0 = int(ty) * TY;
+    // (fewer than 2^23 tiles per residue: the float quotient is at most one off)
+    int ty = __float2int_rz(__fdividef(float(tile), float(g.tiles_x)));
+    int tx = int(tile) - ty * g.tiles_x;
+    if (tx < 0) {
+        --ty;
+        tx += g.tiles_x;
+    } else if (tx >= g.tiles_x) {
+        ++ty;
+        tx -= g.tiles_x;
+    }
+    i0 = tx * TX;
+    j0 = ty * TY;
 }
 
 // The same tile from a 2-D grid (level_grid), without the division.
@@ -1005,17 +1014,24 @@ __global__ void __launch_bounds__(kLvTX* kLvRows, RefOcc<R>::kCtas)
     }
 }
 
-__host__ __device__ inline LevelGeom level_geom(int w, int h, int s, int R)
+// Geometry of the level of stride 2^lg for tiles of R rows per thread.
+__host__ __device__ inline LevelGeom level_geom_lg(int w, int h, int lg, int R)
 {
     LevelGeom g;
-    g.s = s;
-    g.lg = 0;
-    while ((1 << g.lg) < s) ++g.lg;
-    g.sub_w = (w + s - 1) / s;
-    g.sub_h = (h + s - 1) / s;
+    g.s = 1 << lg;
+    g.lg = lg;
+    g.sub_w = (w + g.s - 1) >> lg;
+    g.sub_h = (h + g.s - 1) >> lg;
     g.tiles_x = (g.sub_w + kLvTX - 1) / kLvTX;
     g.tiles_y = (g.sub_h + kLvRows * R - 1) / (kLvRows * R);
     return g;
+}
+
+__host__ __device__ inline LevelGeom level_geom(int w, int h, int s, int R)
+{
+    int lg = 0;
+    while ((1 << lg) < s) ++lg;
+    return level_geom_lg(w, h, lg, R);
 }
 
 __host__ __device__ inline unsigned level_blocks(const LevelGeom& g)

@@ -351,13 +351,14 @@ void launch_stage_kernels(tg_svgf_server* sv, int k, const std::vector<int>& gri
 {
     cudaStream_t st = sv->s_comp;
     cudaMemcpyAsync(sv->d_table[k], sv->h_table[k], sv->tbytes, cudaMemcpyHostToDevice, st);
+    const BatchParams bp = batch_params(sv->d.params, sigma_n_squarings(sv->d.params.sigma_n));
     for (size_t g = 0; g < grids.size(); ++g) {
         if (grids[g] <= 0) continue;
         const char* tab = sv->d_table[k];
         if (g < 2) {
             auto p16 = g == 0 ? k_ms_pixel<ST_FP16, 0> : k_ms_pixel<ST_FP16, 1>;
             auto p32 = g == 0 ? k_ms_pixel<ST_FP32, 0> : k_ms_pixel<ST_FP32, 1>;
-            launch_chain(sv->f16 ? p16 : p32, dim3(grids[g]), pixel_block(int(g)), st, tab, sv->cap);
+            launch_chain(sv->f16 ? p16 : p32, dim3(grids[g]), pixel_block(int(g)), st, tab, sv->cap, bp);
         } else {
             // level 0 stages from the planes, the last level writes only colour
             const int L = int(g) - 2;
@@ -366,7 +367,8 @@ void launch_stage_kernels(tg_svgf_server* sv, int k, const std::vector<int>& gri
                           : (var ? k_ms_level_tma<ST_FP16, kR, true, false> : k_ms_level_tma<ST_FP16, kR, false, false>);
             auto k32 = pl ? k_ms_level_tma<ST_FP32, kR, true, true>
                           : (var ? k_ms_level_tma<ST_FP32, kR, true, false> : k_ms_level_tma<ST_FP32, kR, false, false>);
-            launch_chain(sv->f16 ? k16 : k32, dim3(grids[g]), dim3(kLvTX, kLvRows), st, tab, sv->cap, L, sv->stage_maps[L]);
+            launch_chain(sv->f16 ? k16 : k32, dim3(grids[g]), dim3(kLvTX, kLvRows), st, tab, sv->cap, L, bp,
+                         sv->stage_maps[L]);
         }
     }
 }
