@@ -196,7 +196,7 @@ template <int ST, int R> struct CentrePre {
 
 // IN: the CTA's tile, its halo and every centre's 3x3 neighbourhood lie inside
 // the image (tile_interior), so no access needs a bounds test.
-template <int ST, int R, bool IN>
+template <int ST, int R, bool PL, bool IN>
 __device__ __forceinline__ void level_prefetch(const FullArgs& a, const LevelArgs& lv, int s, int ra, int rb, int i0,
                                                int j0, CentrePre<ST, R>& pre)
 {
@@ -222,6 +222,17 @@ __device__ __forceinline__ void level_prefetch(const FullArgs& a, const LevelArg
         rowf[f] = ((t & m) << lg) * P + (t >> lg) * pw + j_base;
     }
     const Rec::var_t* vp = Rec::var_ptr(lv.col_src, lv.var_off);
+    // level 0: the thread's neighbourhoods overlap, R + 2 rows of three
+    float v0[PL ? R + 2 : 1][3];
+    if constexpr (PL) {
+#pragma unroll
+        for (int f = 0; f < R + 2; ++f) {
+            const int y = j0 + int(threadIdx.y) * R + f - 1;
+            const bool oy = IN || unsigned(y) < unsigned(a.h);
+#pragma unroll
+            for (int e = 0; e < 3; ++e) v0[f][e] = (oy && cxv[e]) ? Rec::var_at(vp, y * a.w + cx + e - 1) : 0.f;
+        }
+    }
 #pragma unroll
     for (int k = 0; k < R; ++k) {
         const int y = rb + s * (j0 + int(threadIdx.y) * R + k);
@@ -232,7 +243,10 @@ __device__ __forceinline__ void level_prefetch(const FullArgs& a, const LevelArg
             const bool oy = pre.valid[k] && (IN || unsigned(y + f - 1) < unsigned(a.h));
 #pragma unroll
             for (int e = 0; e < 3; ++e)
-                pre.vn9[k][f * 3 + e] = (oy && cxv[e]) ? Rec::var_at(vp, rowf[f] + k * pw + cxo[e]) : 0.f;
+                if constexpr (PL)
+                    pre.vn9[k][f * 3 + e] = v0[k + f][e];
+                else
+                    pre.vn9[k][f * 3 + e] = (oy && cxv[e]) ? Rec::var_at(vp, rowf[f] + k * pw + cxo[e]) : 0.f;
         }
     }
 }
@@ -420,7 +434,7 @@ __device__ __forceinline__ void level_tile_body(const FullArgs& a, const LevelAr
     typedef LevelTile<R> T;
     const int s = g.s;
     CentrePre<ST, R> pre;
-    level_prefetch<ST, R, IN>(a, lv, s, ra, rb, i0, j0, pre);
+    level_prefetch<ST, R, PL, IN>(a, lv, s, ra, rb, i0, j0, pre);
     const Rec::rec_t* src = static_cast<const Rec::rec_t*>(lv.col_src);
     const int pw = lv.lin.pw, P = lv.lin.pw * lv.lin.ph;
     const int plane = ((rb << lv.lin.lg) + ra) * P;
@@ -557,7 +571,7 @@ __device__ __forceinline__ void tma_tile_body(const FullArgs& a, const LevelArgs
     constexpr int kCells = (T::N + kThreads - 1) / kThreads;
     const int s = g.s;
     CentrePre<ST, R> pre;
-    level_prefetch<ST, R, IN>(a, lv, s, ra, rb, i0, j0, pre);
+    level_prefetch<ST, R, PL, IN>(a, lv, s, ra, rb, i0, j0, pre);
     // PL: the staged cells' variances (the plane is row-major at level 0)
     float cv[PL ? kCells : 1];
     if constexpr (PL) {
