@@ -1,8 +1,9 @@
-"""The a-trous kernels of two and three output rows per thread compute the same: equal bits (tolerance 0).
+"""The a-trous kernels of one, two and three output rows per thread compute the same: equal bits (tolerance 0).
 
-FULL: the TMA kernels (three rows at the last level, and at every level of a large frame) against the plain-load
-kernels (two rows).  REF_EXACT: the handle's chain (three rows from about 0.6 Mpx) against the chain of the entry
-point without allocation (two rows).  Sizes leave remainders of the 12- and 8-row tiles and of the residue planes.
+FULL: the TMA kernels (one row for small frames, two at 385x211, three at the last level of others and at every level
+of a large frame) against the plain-load kernels (two rows).  REF_EXACT: the handle's chain (three rows from about
+0.6 Mpx) against the chain of the entry point without allocation (two rows).  Sizes leave remainders of the 12- and
+8-row tiles and of the residue planes.
 """
 import os
 import sys
@@ -32,7 +33,7 @@ def frames(w, h, half, n, dev):
         yield d
 
 
-@pytest.mark.parametrize("wh", [(1, 1), (33, 13), (70, 25), (96, 61), (640, 361), (3842, 1213)])
+@pytest.mark.parametrize("wh", [(1, 1), (33, 13), (70, 25), (96, 61), (385, 211), (640, 361), (3842, 1213)])
 @pytest.mark.parametrize("half", [False, True])
 def test_full_rows(cuda_dev, wh, half):
     w, h = wh

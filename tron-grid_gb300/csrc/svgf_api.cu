@@ -209,9 +209,7 @@ LevelTmaFn level_tma_kernel(bool f16, bool pl, bool last, int rows)
 {
     if (rows == 3) return f16 ? level_tma_kernel_r<ST_FP16, 3>(pl, last) : level_tma_kernel_r<ST_FP32, 3>(pl, last);
     if (rows == 1) return f16 ? level_tma_kernel_r<ST_FP16, 1>(pl, last) : level_tma_kernel_r<ST_FP32, 1>(pl, last);
-    // (two rows: never the last level, level_rows)
-    if (f16) return pl ? k_full_level_tma<ST_FP16, 2, true, true> : k_full_level_tma<ST_FP16, 2, true, false>;
-    return pl ? k_full_level_tma<ST_FP32, 2, true, true> : k_full_level_tma<ST_FP32, 2, true, false>;
+    return f16 ? level_tma_kernel_r<ST_FP16, 2>(pl, last) : level_tma_kernel_r<ST_FP32, 2>(pl, last);
 }
 template <bool PL> LevelTiledFn level_tiled_kernel(bool f16, bool last)
 {
@@ -662,7 +660,7 @@ int launch_frame(tg_svgf* s, const tg_svgf_inputs* in, const tg_svgf_outputs* ou
         a.tc = s->tc;
         a.grad = s->grad;
         a.fb_flags = s->fb_flags;
-        a.fb_count = s->d_err + 1;
+        a.fb_count = variance_list(int(grd.x * grd.y), s->sms) ? s->d_err + 1 : nullptr;
         a.err = s->d_err;
         a.alpha = s->p.alpha;
         a.alpha_m = s->p.moments_alpha;
@@ -689,8 +687,7 @@ int launch_frame(tg_svgf* s, const tg_svgf_inputs* in, const tg_svgf_outputs* ou
         });
         // variance: the block flags; the flagged blocks' short-history pixels (data-dependent, not counted)
         launch(s, stream, F_FULL_VARIANCE, double(fb_flags_bytes_of(s->w, s->h)), [&] {
-            const int vg = variance_list_grid(int(grd.x * grd.y), s->sms);
-            launch_chain(f16 ? k_full_variance<ST_FP16> : k_full_variance<ST_FP32>, dim3(vg), dim3(kBlockX, kBlockY / kVarR), stream, a);
+            launch_variance(a, f16, int(grd.x * grd.y), s->sms, stream);
         });
         void* src = s->colA;
         void* oth = s->colB;

@@ -79,7 +79,8 @@ struct FullArgs {
     size_t ghalf;           // FP32 records: index of the guide half-plane (16-byte units)
     float2* grad;           // per-pixel depth gradient (written by the temporal kernel), at grad_idx
     // Blocks of 32x4 pixels with a pixel that needs the spatial variance fallback: with a counter, fb_flags lists
-    // their numbers (in any order) and *fb_count is how many; without one (streams of a batch), fb_flags[block] is 1.
+    // their numbers (in any order) and *fb_count is how many; without one (small frames, streams of a batch),
+    // fb_flags[block] is 1.
     int* fb_flags;
     int* fb_count;
     int* err;               // device error word (bounded waits that gave up); may be null
@@ -433,8 +434,8 @@ template <int ST> __global__ void __launch_bounds__(kBlockX* kBlockY, 8) k_full_
                             blockIdx.y * kBlockY + threadIdx.y);
 }
 
-// The listed blocks, one at a time per CTA of one resident wave (kVarCtas per SM).
-// Level 0 clears the counter for the next frame.
+// The listed blocks, one at a time per CTA of one resident wave.  Level 0 clears the
+// counter for the next frame.
 template <int ST> __global__ void __launch_bounds__(kBlockX* kBlockY / kVarR, kVarCtas) k_full_variance(FullArgs a)
 {
     __shared__ VarTile vt;
@@ -446,6 +447,31 @@ template <int ST> __global__ void __launch_bounds__(kBlockX* kBlockY / kVarR, kV
     }
 }
 
-__host__ inline int variance_list_grid(int blocks, int sms) { return blocks < kVarCtas * sms ? blocks : kVarCtas * sms; }
+// A small frame: one CTA per pixel block, which looks at its own flag.  The frame
+// waits for one block's time here, which one pixel per thread halves (383x209 right
+// after a cut 48.2 us per frame against 50.5), and which the list's counter and entry
+// would put two loads in front of (steady 40.0 against 41.5, 512x288 43.5 against 44.4).
+constexpr int kVarSmallCtas = 8;
+template <int ST> __global__ void __launch_bounds__(kBlockX* kBlockY, kVarSmallCtas) k_full_variance_small(FullArgs a)
+{
+    __shared__ VarTile vt;
+    pdl_begin();
+    const int tx = (a.w + kBlockX - 1) / kBlockX, b = blockIdx.x;
+    if (__ldcg(a.fb_flags + b)) full_variance_tile<ST, 1>(a, (b % tx) * kBlockX, (b / tx) * kBlockY, vt);
+}
+
+// Whether the estimate over a frame of `blocks` pixel blocks takes a list of them
+// (more blocks than one wave of the small form holds) or flags.
+inline bool variance_list(int blocks, int sms) { return blocks > kVarSmallCtas * sms; }
+
+inline cudaError_t launch_variance(const FullArgs& a, bool f16, int blocks, int sms, cudaStream_t st)
+{
+    if (!variance_list(blocks, sms))
+        return launch_chain(f16 ? k_full_variance_small<ST_FP16> : k_full_variance_small<ST_FP32>, dim3(blocks),
+                            dim3(kBlockX, kBlockY), st, a);
+    const int wave = kVarCtas * sms;
+    return launch_chain(f16 ? k_full_variance<ST_FP16> : k_full_variance<ST_FP32>, dim3(blocks < wave ? blocks : wave),
+                        dim3(kBlockX, kBlockY / kVarR), st, a);
+}
 
 } // namespace tg

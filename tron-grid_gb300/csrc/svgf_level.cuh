@@ -77,16 +77,20 @@ template <int R> struct LevelOcc {
 // 50 / 56 (7 waves).  The last level writes only colour and is bound by its
 // scattered stores more than by its registers: three rows are faster from
 // 640x360 (12.8 against 13.2 us) to 3840x2160 (207 against 222).
-// A frame whose one-row tiles fit a single wave takes one row: its levels are
-// one tile's latency each (160x90 26.8 us per frame on the GPU against 33.9 with
-// two and three rows, 480x270 46.8 against 49.8; 640x360, 1800 tiles, 66.5
-// against 62.0).
+// A frame whose one-row tiles fit a single wave has levels of one or a few tiles'
+// latency each, and takes one row: 23.4 us per frame against 28.2 with two at
+// 160x90, 42.3 against 45.5 at 352x288, 43.5 against 47.8 at 512x288 (640x360,
+// 1800 tiles, 66.5 against 62.0).  Four and five one-row tiles on the busiest SM
+// are the exception, which two or three two-row tiles replace: 37.7 us with two
+// rows against 40.0 with one at 383x209, 40.2 against 41.1 at 400x225 (three
+// tiles, 320x180, 35.3 against 34.8; six, 448x252, 43.3 against 41.8).
 __host__ inline int level_rows(int w, int h, bool last)
 {
     auto tiles = [&](int rows) {
         return (long long)((w + kLvTX - 1) / kLvTX) * ((h + rows * kLvRows - 1) / (rows * kLvRows));
     };
-    if (tiles(1) <= 8 * 152) return 1;
+    const long long deep = (tiles(1) + 151) / 152;
+    if (deep <= 8) return deep == 4 || deep == 5 ? 2 : 1;
     return last || tiles(3) >= 16 * 5 * 152 ? 3 : 2;
 }
 

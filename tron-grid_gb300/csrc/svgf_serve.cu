@@ -452,10 +452,9 @@ void launch_plain(tg_svgf_server* sv, Sess& s)
     const dim3 blk(kBlockX, kBlockY);
     const dim3 grd((s.w + kBlockX - 1) / kBlockX, (s.h + kBlockY - 1) / kBlockY);
     cudaStream_t st = sv->s_comp;
-    a.fb_count = sv->d_fb;  // (launches are ordered on s_comp)
-    const int vg = variance_list_grid(int(grd.x * grd.y), sv->sm_count);
+    a.fb_count = variance_list(int(grd.x * grd.y), sv->sm_count) ? sv->d_fb : nullptr;  // (ordered on s_comp)
     launch_chain(sv->f16 ? k_full_temporal<ST_FP16> : k_full_temporal<ST_FP32>, grd, blk, st, a);
-    launch_chain(sv->f16 ? k_full_variance<ST_FP16> : k_full_variance<ST_FP32>, dim3(vg), dim3(kBlockX, kBlockY / kVarR), st, a);
+    launch_variance(a, sv->f16, int(grd.x * grd.y), sv->sm_count, st);
     void* src = s.colA;
     void* oth = s.colB;
     for (int lv = 0; lv < sv->d.params.levels; ++lv) {
