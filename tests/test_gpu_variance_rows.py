@@ -1,4 +1,4 @@
-"""The spatial variance estimate of single streams (small frames: a CTA per flagged block; others, here 577x290: two
+"""The spatial variance estimate of single streams (small frames: a CTA per flagged block; others, here 1282x730: two
 pixels per thread over listed blocks) against the persistent batch kernel (one pixel per thread over flagged blocks):
 equal bits (tolerance 0).
 
@@ -23,7 +23,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("half", [False, True])
 def test_list_equals_flags(cuda_dev, half):
-    sizes = [(1, 1), (31, 3), (33, 5), (70, 7), (64, 130), (577, 290)]
+    sizes = [(1, 1), (31, 3), (33, 5), (70, 7), (64, 130), (577, 290), (1282, 730)]
     st = tg.STORAGE_FP16 if half else tg.STORAGE_FP32
     b = Batch(sizes, storage=st, strategy=L.BATCH_PERSISTENT)
     dens = [tg.Denoiser(w, h, storage=st) for w, h in sizes]

@@ -79,7 +79,7 @@ struct FullArgs {
     size_t ghalf;           // FP32 records: index of the guide half-plane (16-byte units)
     float2* grad;           // per-pixel depth gradient (written by the temporal kernel), at grad_idx
     // Blocks of 32x4 pixels with a pixel that needs the spatial variance fallback: with a counter, fb_flags lists
-    // their numbers (in any order) and *fb_count is how many; without one (small frames, streams of a batch),
+    // their numbers (in any order) and *fb_count is how many; without one (variance_list, streams of a batch),
     // fb_flags[block] is 1.
     int* fb_flags;
     int* fb_count;
@@ -434,25 +434,25 @@ template <int ST> __global__ void __launch_bounds__(kBlockX* kBlockY, 8) k_full_
                             blockIdx.y * kBlockY + threadIdx.y);
 }
 
-// The listed blocks, one at a time per CTA of one resident wave.  Level 0 clears the
-// counter for the next frame.
+// The listed blocks, one at a time per CTA of one resident wave.  The list is in the
+// order that the temporal pass's blocks finished; when it holds every block (the
+// frames after a cut) they are taken in image order instead, whose neighbours share
+// their halos in L1 and L2.  Level 0 clears the counter for the next frame.
 template <int ST> __global__ void __launch_bounds__(kBlockX* kBlockY / kVarR, kVarCtas) k_full_variance(FullArgs a)
 {
     __shared__ VarTile vt;
     pdl_begin();
-    const int tx = (a.w + kBlockX - 1) / kBlockX, n = min(__ldcg(a.fb_count), pixel_blocks(a));
+    const int tx = (a.w + kBlockX - 1) / kBlockX, all = pixel_blocks(a), n = min(__ldcg(a.fb_count), all);
     for (int e = blockIdx.x; e < n; e += gridDim.x) {
-        const int b = __ldcg(a.fb_flags + e);
+        const int b = n == all ? e : __ldcg(a.fb_flags + e);
         full_variance_tile<ST, kVarR>(a, (b % tx) * kBlockX, (b / tx) * kBlockY, vt);
     }
 }
 
-// A small frame: one CTA per pixel block, which looks at its own flag.  The frame
-// waits for one block's time here, which one pixel per thread halves (383x209 right
-// after a cut 48.2 us per frame against 50.5), and which the list's counter and entry
-// would put two loads in front of (steady 40.0 against 41.5, 512x288 43.5 against 44.4).
-constexpr int kVarSmallCtas = 8;
-template <int ST> __global__ void __launch_bounds__(kBlockX* kBlockY, kVarSmallCtas) k_full_variance_small(FullArgs a)
+// One CTA per pixel block, which looks at its own flag: no counter and no entry to
+// wait for before the first block, and blocks in image order.  One pixel per thread:
+// the frame waits for one block's time here, which two per thread would double.
+template <int ST> __global__ void __launch_bounds__(kBlockX* kBlockY, 8) k_full_variance_flags(FullArgs a)
 {
     __shared__ VarTile vt;
     pdl_begin();
@@ -460,14 +460,17 @@ template <int ST> __global__ void __launch_bounds__(kBlockX* kBlockY, kVarSmallC
     if (__ldcg(a.fb_flags + b)) full_variance_tile<ST, 1>(a, (b % tx) * kBlockX, (b / tx) * kBlockY, vt);
 }
 
-// Whether the estimate over a frame of `blocks` pixel blocks takes a list of them
-// (more blocks than one wave of the small form holds) or flags.
-inline bool variance_list(int blocks, int sms) { return blocks > kVarSmallCtas * sms; }
+// Whether the estimate over a frame of `blocks` pixel blocks takes a list of them or
+// flags.  Flags cost a CTA for every block that needs nothing: steady frames
+// of 1280x720 (7200 blocks) take 163 us either way, 1920x1080 331.7 with flags against
+// 326.0 and 3840x2160 1195 against 1154; 960x540 102.7 against 103.9, 564x307 58.8
+// against 61.2, and right after a cut 122.5 against 130.1 and 67.9 against 71.2.
+inline bool variance_list(int blocks, int sms) { return blocks > 48 * sms; }
 
 inline cudaError_t launch_variance(const FullArgs& a, bool f16, int blocks, int sms, cudaStream_t st)
 {
     if (!variance_list(blocks, sms))
-        return launch_chain(f16 ? k_full_variance_small<ST_FP16> : k_full_variance_small<ST_FP32>, dim3(blocks),
+        return launch_chain(f16 ? k_full_variance_flags<ST_FP16> : k_full_variance_flags<ST_FP32>, dim3(blocks),
                             dim3(kBlockX, kBlockY), st, a);
     const int wave = kVarCtas * sms;
     return launch_chain(f16 ? k_full_variance<ST_FP16> : k_full_variance<ST_FP32>, dim3(blocks < wave ? blocks : wave),
