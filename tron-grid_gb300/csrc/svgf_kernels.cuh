@@ -434,23 +434,22 @@ template <int ST> __global__ void __launch_bounds__(kBlockX* kBlockY, 8) k_full_
                             blockIdx.y * kBlockY + threadIdx.y);
 }
 
-// The listed blocks, one at a time per CTA of one resident wave.  The list is in the
-// order that the temporal pass's blocks finished; when it holds every block (the
-// frames after a cut) they are taken in image order instead, whose neighbours share
-// their halos in L1 and L2.  Level 0 clears the counter for the next frame.
+// The listed blocks, one at a time per CTA of one resident wave (taken by ticket
+// instead: 3840x2160 after a cut 1495 against 1520 us, but steady 1920x1080 328.1
+// against 325.9).  Level 0 clears the counter for the next frame.
 template <int ST> __global__ void __launch_bounds__(kBlockX* kBlockY / kVarR, kVarCtas) k_full_variance(FullArgs a)
 {
     __shared__ VarTile vt;
     pdl_begin();
-    const int tx = (a.w + kBlockX - 1) / kBlockX, all = pixel_blocks(a), n = min(__ldcg(a.fb_count), all);
+    const int tx = (a.w + kBlockX - 1) / kBlockX, n = min(__ldcg(a.fb_count), pixel_blocks(a));
     for (int e = blockIdx.x; e < n; e += gridDim.x) {
-        const int b = n == all ? e : __ldcg(a.fb_flags + e);
+        const int b = __ldcg(a.fb_flags + e);
         full_variance_tile<ST, kVarR>(a, (b % tx) * kBlockX, (b / tx) * kBlockY, vt);
     }
 }
 
 // One CTA per pixel block, which looks at its own flag: no counter and no entry to
-// wait for before the first block, and blocks in image order.  One pixel per thread:
+// wait for before the first block.  One pixel per thread:
 // the frame waits for one block's time here, which two per thread would double.
 template <int ST> __global__ void __launch_bounds__(kBlockX* kBlockY, 8) k_full_variance_flags(FullArgs a)
 {
