@@ -239,6 +239,7 @@ struct tg_svgf {
     float2* grad = nullptr;
     int* fb_flags = nullptr;
     int* d_err = nullptr;  // device error word of bounded waits, then (FULL) the counter of fallback blocks
+    bool fb_stale = false; // the counter may hold a failed frame's entries (clear_stale_count)
     int flags = 0;
     bool tma = false;                // a-trous tiles staged by TMA
     int rows[10];                    // output rows per thread of each FULL level's TMA kernel (level_rows)
@@ -489,6 +490,7 @@ int alloc_buffers(tg_svgf* s)
         free_buffers(s);
         return fail(TG_ERR_CUDA, "zeroing the SVGF state failed: %s", cudaGetErrorString(cudaGetLastError()));
     }
+    s->fb_stale = false;
     return TG_OK;
 }
 
@@ -661,6 +663,8 @@ int launch_frame(tg_svgf* s, const tg_svgf_inputs* in, const tg_svgf_outputs* ou
         a.grad = s->grad;
         a.fb_flags = s->fb_flags;
         a.fb_count = variance_list(int(grd.x * grd.y), s->sms) ? s->d_err + 1 : nullptr;
+        if (a.fb_count && clear_stale_count(a.fb_count, s->fb_stale, stream) != cudaSuccess)
+            return fail(TG_ERR_CUDA, "fallback counter clear failed: %s", cudaGetErrorString(cudaGetLastError()));
         a.err = s->d_err;
         a.alpha = s->p.alpha;
         a.alpha_m = s->p.moments_alpha;
@@ -722,7 +726,10 @@ int launch_frame(tg_svgf* s, const tg_svgf_inputs* in, const tg_svgf_outputs* ou
         }
     }
     cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return fail(TG_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+        s->fb_stale = true;
+        return fail(TG_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString(e));
+    }
     s->frame++;
     return TG_OK;
 }

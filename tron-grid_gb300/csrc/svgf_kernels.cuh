@@ -342,7 +342,7 @@ template <int ST> __device__ __forceinline__ void full_temporal_block(const Full
             a.fb_flags[blk] = any;
         else if (any) {
             const int at = atomicAdd(a.fb_count, 1);
-            if (at < pixel_blocks(a)) a.fb_flags[at] = blk;  // (always, unless a frame's launches failed half-way)
+            if (at < pixel_blocks(a)) a.fb_flags[at] = blk;  // (always: the counter is 0 before a frame)
         }
     }
 }
@@ -465,6 +465,21 @@ template <int ST> __global__ void __launch_bounds__(kBlockX* kBlockY, 8) k_full_
 // 326.0 and 3840x2160 1195 against 1154; 960x540 102.7 against 103.9, 564x307 58.8
 // against 61.2, and right after a cut 122.5 against 130.1 and 67.9 against 71.2.
 inline bool variance_list(int blocks, int sms) { return blocks > 48 * sms; }
+
+// The list's counter between frames: level 0 leaves it 0, but a frame of which a
+// launch was rejected may not have got there (`stale`), and the next frame would
+// append to that frame's entries.  Called before such a frame's launches.  A
+// captured frame keeps the clearing in its graph, so the next frame that runs at
+// once still needs its own.
+inline cudaError_t clear_stale_count(int* count, bool& stale, cudaStream_t st)
+{
+    if (!stale) return cudaSuccess;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(st, &cs);
+    if (e == cudaSuccess) e = cudaMemsetAsync(count, 0, sizeof *count, st);
+    if (e == cudaSuccess && cs == cudaStreamCaptureStatusNone) stale = false;
+    return e;
+}
 
 inline cudaError_t launch_variance(const FullArgs& a, bool f16, int blocks, int sms, cudaStream_t st)
 {

@@ -175,7 +175,8 @@ struct tg_svgf_server {
     char* h_table[kMaxInflight] = {};
     int* h_err = nullptr;
     BarrierState* d_bar = nullptr;
-    int* d_fb = nullptr;  // counter of fallback blocks of the plain path
+    int* d_fb = nullptr;   // counter of fallback blocks of the plain path
+    bool fb_stale = false; // it may hold a failed launch's entries, of any session (clear_stale_count)
     cudaGraphExec_t exec[kMaxInflight] = {};
     std::vector<cudaEvent_t> ev_pool;  // completion events, reused
     StageMaps stage_maps[10];          // the stage kernels' maps of the launch being formed (one per level)
@@ -453,6 +454,7 @@ void launch_plain(tg_svgf_server* sv, Sess& s)
     const dim3 grd((s.w + kBlockX - 1) / kBlockX, (s.h + kBlockY - 1) / kBlockY);
     cudaStream_t st = sv->s_comp;
     a.fb_count = variance_list(int(grd.x * grd.y), sv->sm_count) ? sv->d_fb : nullptr;  // (ordered on s_comp)
+    if (a.fb_count && clear_stale_count(a.fb_count, sv->fb_stale, st) != cudaSuccess) return;  // (the caller sees the error)
     launch_chain(sv->f16 ? k_full_temporal<ST_FP16> : k_full_temporal<ST_FP32>, grd, blk, st, a);
     launch_variance(a, sv->f16, int(grd.x * grd.y), sv->sm_count, st);
     void* src = s.colA;
@@ -668,6 +670,7 @@ void scheduler(tg_svgf_server* sv)
         else
             launch_plain(sv, *ss[0]);
         fl->launch_failed = cudaGetLastError() != cudaSuccess;
+        if (fl->launch_failed) sv->fb_stale = true;
         cudaEventRecord(fl->ev_comp, sv->s_comp);
         cudaStreamWaitEvent(sv->s_d2h, fl->ev_comp, 0);
         for (size_t j = 0; j < batch.size(); ++j) {
