@@ -32,7 +32,7 @@ def program(tmp_path_factory):
     return str(exe)
 
 
-@pytest.mark.parametrize("which", ["counter"])
+@pytest.mark.parametrize("which", ["counter", "last"])
 def test_rejected_launch(program, which):
     r = subprocess.run([program, which], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout + r.stderr

@@ -375,6 +375,9 @@ int tg_fog_filter(const tg_fog_filter_params* p, const tg_volume* raw, const tg_
         {k_fog_filter<false, false, uint64_t>, k_fog_filter<false, true, uint64_t>, k_fog_filter<true, false, uint64_t>,
          k_fog_filter<true, true, uint64_t>}};
     const cudaError_t e = launch_chain(fns[wide][2 * r16 + o16], grid, block, s, a);
-    if (e != cudaSuccess) return fail(TG_ERR_CUDA, "fog filter launch failed: %s", cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+        cudaGetLastError();  // (reported here, not by the thread's next call)
+        return fail(TG_ERR_CUDA, "fog filter launch failed: %s", cudaGetErrorString(e));
+    }
     return TG_OK;
 }

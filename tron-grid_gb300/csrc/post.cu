@@ -531,14 +531,20 @@ int tg_post_process(tg_post* s, const tg_image* hdr, const tg_image* out, void* 
         e = launch_chain(k_bloom_down, grid(s->mip[i].w, s->mip[i].h), blk, cs, s->mip[i - 1], s->mip[i]);
     for (int i = s->n - 2; i >= 0 && e == cudaSuccess; --i)
         e = launch_chain(k_bloom_up, grid((s->mip[i].w + 1) / 2, (s->mip[i].h + 1) / 2), blk, cs, s->mip[i + 1], s->mip[i]);
-    if (e != cudaSuccess) return fail(TG_ERR_CUDA, "bloom launch failed: %s", cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+        cudaGetLastError();  // (reported here, not by the thread's next call)
+        return fail(TG_ERR_CUDA, "bloom launch failed: %s", cudaGetErrorString(e));
+    }
     typedef void (*PostFn)(const char*, long long, char*, long long, int, int, Mip, float, float, float, int);
     static const PostFn fns[2][3] = {{k_post<false, OUT_BGRA8>, k_post<false, OUT_RGBA8>, k_post<false, OUT_RGBA32F>},
                                      {k_post<true, OUT_BGRA8>, k_post<true, OUT_RGBA8>, k_post<true, OUT_RGBA32F>}};
     const int of = out->format == TG_FMT_BGRA8 ? OUT_BGRA8 : out->format == TG_FMT_RGBA8 ? OUT_RGBA8 : OUT_RGBA32F;
     e = launch_chain(fns[h16][of], grid((W + 1) / 2, H), blk, cs, hb, hp, static_cast<char*>(out->ptr), op, W, H, s->mip[0],
                      s->p.bloom_strength, 1.0f / float(W), 1.0f / float(H), vec);
-    if (e != cudaSuccess) return fail(TG_ERR_CUDA, "post-process launch failed: %s", cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return fail(TG_ERR_CUDA, "post-process launch failed: %s", cudaGetErrorString(e));
+    }
     return TG_OK;
 }
 

@@ -358,7 +358,10 @@ int run_step(tg_svgf_batch* b, uint32_t n, const uint32_t* ids, const tg_svgf_in
         e = cudaGraphLaunch(b->exec[k], stream);
     else
         e = launch_step(b, k, stream);
-    if (e != cudaSuccess) return fail(TG_ERR_CUDA, "batch step launch failed: %s", cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+        cudaGetLastError();  // (reported here, not by the thread's next call)
+        return fail(TG_ERR_CUDA, "batch step launch failed: %s", cudaGetErrorString(e));
+    }
     if (cudaEventRecord(b->table_free[k], stream) != cudaSuccess) return fail(TG_ERR_CUDA, "event record failed");
     b->table_used[k] = true;
     b->tbuf ^= 1;
