@@ -53,3 +53,19 @@ def test_volumes_beyond_32_bit_offsets(cuda_dev, which):
     far.copy_(raw if which == "raw" else hist)
     got = tg.fog_filter(p, far if which == "raw" else raw, far if which == "history" else hist, out=torch.empty_like(raw))
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("base", [0, (1 << 23) - 200, (1 << 24) - 200])
+def test_mean_of_subnormal_sums(cuda_dev, base):
+    """Boxes of six whose sums are base + 1 .. base + 408 units of 2^-149: below 2^-125 their quotients are subnormal,
+    where a third of a unit and a half of one are both met.  Equals the oracle bit for bit (tolerance 0)."""
+    w, h, d = 33, 9, 17
+    units = np.zeros((d, h, w, 4), np.uint32)  # a float32 of these bits is that many units of 2^-149, up to 2^24
+    units[:, 1::3, ::w - 1, :] = base + 1 + np.arange(d * 3 * 2 * 4, dtype=np.uint32).reshape(d, 3, 2, 4)
+    raw = units.view(np.float32)
+    raw[1::2] *= -1.0
+    args = fog_scene.FogScene(fog_scene.FogSpec(width=w, height=h, depth=d)).param_args(0)
+    out = tg.fog_filter(tg.fog_params(**args), torch.from_numpy(raw).to(cuda_dev),
+                        torch.zeros((d, h, w, 4), device=cuda_dev))
+    want = oracle.fog_filter(oracle.fog_param_block(**args), raw, np.zeros_like(raw), fp16_store=False)
+    np.testing.assert_array_equal(out.cpu().numpy(), want)

@@ -104,15 +104,19 @@ __device__ __forceinline__ void mat_vec(const float* m, float x, float y, float 
     for (int r = 0; r < 4; ++r) o[r] = add(add(add(mul(m[r], x), mul(m[4 + r], y)), mul(m[8 + r], z)), mul(m[12 + r], w));
 }
 
-// x / y by the correctly rounded reciprocal r of y: one residual step is exact
-// for the box counts (every binary32 significand over 3, 6 and 9 was checked;
-// 1, 2 and 4 are exact), two steps for any divisor.  |x| < 2^100 and x / y far
+// x / y by the correctly rounded reciprocal r of y, |x| < 2^100.  One residual
+// step is exact for the box counts (every binary32 significand over 3, 6 and 9 was
+// checked; 1, 2 and 4 are exact), for subnormal quotients too but over 6, where a
+// quotient can lie half-way between two subnormals and the step does not keep the
+// tie: every x below 2^-99 was checked, the last wrong one lies below 2^-125
+// (count_is_subnormal).  Two steps are exact for any divisor while x / y is far
 // from the subnormals, or x = 0.
 __device__ __forceinline__ float div_count(float x, float y, float r)
 {
     const float q = mul(x, r);
     return __fmaf_rn(__fmaf_rn(-q, y, x), r, q);
 }
+__device__ __forceinline__ bool count_is_subnormal(float x) { return x != 0.f && fabsf(x) < 4.7019774e-38f; }  // 2^-124
 __device__ __forceinline__ float div_by(float x, float y, float r)
 {
     const float q = div_count(x, y, r);
@@ -227,7 +231,10 @@ __global__ void __launch_bounds__(kFogTX* kFogTY, 9) k_fog_filter(const FogArgs 
                 s = make_float4(add(s.x, q.x), add(s.y, q.y), add(s.z, q.z), add(s.w, q.w));
             }
         float4 res;
-        if (fmaxf(fmaxf(fabsf(s.x), fabsf(s.y)), fmaxf(fabsf(s.z), fabsf(s.w))) < kDivMax)
+        bool plain = !(fmaxf(fmaxf(fabsf(s.x), fabsf(s.y)), fmaxf(fabsf(s.z), fabsf(s.w))) < kDivMax);
+        if (!RAW16 && cnt == 6.f)  // (sums of binary16 texels are multiples of 2^-24)
+            plain |= count_is_subnormal(s.x) || count_is_subnormal(s.y) || count_is_subnormal(s.z) || count_is_subnormal(s.w);
+        if (!plain)
             res = make_float4(div_count(s.x, cnt, rcnt), div_count(s.y, cnt, rcnt), div_count(s.z, cnt, rcnt),
                               div_count(s.w, cnt, rcnt));
         else
