@@ -35,3 +35,23 @@ def test_streams_match_handles(cuda_dev, sizes, pick):
     b.close()
     for d in dens.values():
         d.close()
+
+
+@pytest.mark.parametrize("n", [256, 257])
+def test_lookup_over_many_streams(cuda_dev, n):
+    """A step of 256 streams is the last that looks a tile's stream up by ballots; one of 257 searches by halves."""
+    sizes = [(17 + k % 40, 5 + k % 4) for k in range(n)]
+    b = Batch(sizes, storage=tg.STORAGE_FP32)
+    picks = [0, 31, 32, 33, 128, 254, n - 1]
+    dens = {k: tg.Denoiser(*sizes[k]) for k in picks}
+    scenes = [scene.PlaneScene(scene.pan_with_disocclusion(*s, seed=k), cuda_dev) for k, s in enumerate(sizes)]
+    for t in (29, 30):
+        fr = [{q: v for q, v in sc.frame(t).items() if q in ("radiance", "depth", "normal", "motion")} for sc in scenes]
+        outs = [torch.empty((h, w, 4), device=cuda_dev) for w, h in sizes]
+        b.denoise(list(range(n)), fr, outs)
+        b.synchronize()
+        for k in picks:
+            assert torch.equal(dens[k].denoise(**fr[k]), outs[k])
+    b.close()
+    for d in dens.values():
+        d.close()

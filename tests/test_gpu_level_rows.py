@@ -8,16 +8,19 @@ of a large frame) against the plain-load kernels (two rows).  REF_EXACT: the han
 import os
 import sys
 
+import numpy as np
 import pytest
 import torch
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 sys.path.insert(0, ROOT)
 
+import oracle  # noqa: E402
 import tron_grid_gb300 as tg  # noqa: E402
 from tron_grid_gb300 import _lib as L  # noqa: E402
 from tron_grid_gb300 import scene  # noqa: E402
 from tron_grid_gb300.svgf import image  # noqa: E402
+from tests.helpers import REL_TOL, rel_err  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 
@@ -73,3 +76,24 @@ def test_ref_rows(cuda_dev, wh, half):
         got = den.denoise(f["radiance"], out=torch.empty_like(want))
         assert torch.equal(got, want)
     den.close()
+
+
+@pytest.mark.parametrize("wh", [(1281, 721), (1284, 723)])
+@pytest.mark.parametrize("half", [False, True])
+def test_ref_three_rows(cuda_dev, wh, half):
+    """Chains of three rows (10 * 152 tiles of 32 x 12 and more) in both storage forms: staged by TMA and by plain loads
+    the bits are equal, and equal to the oracle's within the parity tests' tolerance (binary16 images: one step of the
+    store in each of the three passes, 2^-10 relative each)."""
+    w, h = wh
+    assert ((w + 31) // 32) * ((h + 11) // 12) >= 10 * 152
+    st, dt = (tg.STORAGE_FP16, torch.float16) if half else (tg.STORAGE_FP32, torch.float32)
+    a = tg.Denoiser(w, h, mode=tg.MODE_REF_EXACT, storage=st)
+    b = tg.Denoiser(w, h, mode=tg.MODE_REF_EXACT, storage=st, flags=L.FLAG_NO_TMA)
+    mom = np.zeros((h, w, 2), np.float32)
+    for f in frames(w, h, half, 2, cuda_dev):
+        x, y = (d.denoise(f["radiance"], out=torch.empty((h, w, 4), dtype=dt, device=cuda_dev)) for d in (a, b))
+        assert torch.equal(x, y)
+        want, mom = oracle.ref_frame(f["radiance"].float().cpu().numpy(), mom, fp16_store=half)
+        assert rel_err(x.float().cpu().numpy(), want).max() <= (3 * 2.0 ** -10 if half else REL_TOL)
+    a.close()
+    b.close()
