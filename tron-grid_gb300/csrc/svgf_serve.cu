@@ -825,7 +825,7 @@ int tg_svgf_server_create(const tg_svgf_server_desc* d, tg_svgf_server** out)
                 return bail(fail(TG_ERR_OOM, "work table allocation failed"));
         if (cudaHostAlloc(reinterpret_cast<void**>(&sv->h_err), kMaxInflight * sizeof(int), cudaHostAllocDefault) !=
                 cudaSuccess ||
-            cudaMalloc(&sv->d_bar, sizeof(BarrierState) + sizeof(int)) != cudaSuccess)
+            cudaMalloc(&sv->d_bar, sizeof(BarrierState)) != cudaSuccess)
             return bail(fail(TG_ERR_OOM, "barrier allocation failed"));
         for (int k = 0; k < kMaxInflight; ++k) sv->h_err[k] = 0;
     }
