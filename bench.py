@@ -1094,6 +1094,28 @@ def run_reference(args, rank, world):
     return res
 
 
+def printed(res):
+    """What the one line on stdout holds, and the per-frame lists it leaves out (printed to stderr).  The line has to
+    stay short enough to be read back whole: the lists alone were more than half of it.  The figures inside the
+    sections are cut to six digits; the line's own (value, ms_per_step, ...) are not."""
+    lists = {}
+
+    def short(v, path):
+        if isinstance(v, dict):
+            out = {}
+            for k, x in v.items():
+                if k == "per_frame":
+                    lists["/".join(path)] = x
+                else:
+                    out[k] = short(x, (*path, k))
+            return out
+        if isinstance(v, (list, tuple)):
+            return [short(x, path) for x in v]
+        return float(f"{v:.6g}") if isinstance(v, float) and len(path) > 1 else v
+
+    return short(res, ()), lists
+
+
 def main(argv=None):
     args = parse_args(argv)
     if args.only is not None:
@@ -1114,6 +1136,10 @@ def main(argv=None):
     else:
         res = run_tg(args, rank, world, local)
     if rank == 0 and res is not None:
+        if args.impl != "reference":
+            res, lists = printed(res)
+            if lists:
+                print(json.dumps({"per_frame": lists}), file=sys.stderr, flush=True)
         print(json.dumps(res), flush=True)
     if world > 1:
         import torch.distributed as dist

@@ -68,3 +68,26 @@ def test_timed_window_holds_the_disocclusion():
     w0, t0 = bench.first_frames(120, 5, 60)
     assert t0 == 5 and w0 == 0
     assert "20..39" in bench.window_text(20, 20, 60)
+
+
+def test_line_leaves_the_per_frame_lists_to_stderr(monkeypatch, capsys):
+    """One JSON line on stdout without the accuracy report's 60-entry lists, which go to stderr whole; the headline's
+    figures are printed in full."""
+    sys.path.insert(0, ROOT)
+    import bench
+
+    lists = {k: [0.1 + i for i in range(60)] for k in ("max_abs", "max_rel", "rel_l2", "psnr_db")}
+    forms = ("fp32", "fp16", "fp16_images", "fp16_out16")
+    res = {"metric": bench.METRIC, "value": 835.1234567890123, "ms_per_step": 1.1974279876543211, "e2e": None,
+           "roofline": {"frac": 0.5123456789, "kernel": "full_level"},
+           "accuracy": {"workload": "w", **{f: {"max_abs": 1.23456789e-05, "per_frame": lists} for f in forms}}}
+    monkeypatch.setattr(bench, "run_tg", lambda *a: res)
+    monkeypatch.setattr(bench, "dist_setup", lambda: (0, 1, 0))
+    bench.main(["--steps", "2"])
+    got = capsys.readouterr()
+    assert got.out.count("\n") == 1 and len(got.out) < 1024
+    d = json.loads(got.out)
+    assert d["value"] == res["value"] and d["ms_per_step"] == res["ms_per_step"] and d["e2e"] is None
+    assert d["roofline"] == {"frac": 0.512346, "kernel": "full_level"}
+    assert d["accuracy"] == {"workload": "w", **{f: {"max_abs": 1.23457e-05} for f in forms}}
+    assert json.loads(got.err)["per_frame"] == {f"accuracy/{f}": lists for f in forms}
