@@ -9,7 +9,7 @@
 // and each thread places its froxel centre on its ray, projects it into the
 // previous frame and fetches the history trilinearly.
 //
-// What bounds it: FP32 issue (about 480 instructions per froxel, the unfused
+// What bounds it: FP32 issue (510 instructions per froxel, the unfused
 // interpolation of eight texels the largest part).  The compulsory traffic of a
 // 320x180x64 rgba16f pass (88 MB, L2-resident) is 13 us of the 6.8 TB/s a copy
 // reaches.  Measured there, with history: 79.9 us with two barriers per slice and a

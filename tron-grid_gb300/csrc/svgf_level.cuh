@@ -73,8 +73,8 @@ template <int R> struct LevelOcc {
 // fewer instructions and a fifth less shared-memory traffic per output, but only
 // five CTAs are resident, so a level of few waves loses more to its last one:
 // 3840x2160 187 / 174 / 180 / 190 us for levels 0 to 3 against 193 / 180 / 183 /
-// 188 with two rows (28 waves), 1920x1080 52 / 49 / 53.5 / 59 against 52 / 49 /
-// 50 / 56 (7 waves).  The last level writes only colour and is bound by its
+// 188 with two rows (28 waves; level 3, 1% slower with three, follows the others),
+// 1920x1080 52 / 49 / 53.5 / 59 against 52 / 49 / 50 / 56 (7 waves).  The last level writes only colour and is bound by its
 // scattered stores more than by its registers: three rows are faster from
 // 640x360 (12.8 against 13.2 us) to 3840x2160 (207 against 222).
 // A frame whose one-row tiles fit a single wave has levels of one or a few tiles'
@@ -84,6 +84,7 @@ template <int R> struct LevelOcc {
 // are the exception, which two or three two-row tiles replace: 37.7 us with two
 // rows against 40.0 with one at 383x209, 40.2 against 41.1 at 400x225 (three
 // tiles, 320x180, 35.3 against 34.8; six, 448x252, 43.3 against 41.8).
+// (152: the SMs of a GB300, here and in ref_rows.)
 __host__ inline int level_rows(int w, int h, bool last)
 {
     auto tiles = [&](int rows) {
@@ -907,7 +908,8 @@ template <int R> struct RefOcc {
 // Output rows per thread of a REF_EXACT chain: three share each staged texel and
 // the per-thread work among more outputs (3840x2160, binary16 images: 223 us
 // against 238 with two rows), two leave a small frame more CTAs (640x360: 19
-// against 22 us; even at 1280x720).
+// against 22 us).  The line is one full wave of three-row CTAs; the two are even at
+// 1280x720, where they make 1.58 and 1.97 waves.
 __host__ inline int ref_rows(int w, int h)
 {
     const long long tiles = (long long)((w + kLvTX - 1) / kLvTX) * ((h + 3 * kLvRows - 1) / (3 * kLvRows));
